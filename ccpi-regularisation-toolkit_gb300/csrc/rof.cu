@@ -148,6 +148,8 @@ int rof_run(const float* f, float* u_out, const float* lam_arr, float lam, int i
             const Dims& d, cudaStream_t s, float* info, const float* u_init) {
     CILREG_RANGE("cilreg ROF-TV");
     CILREG_TRY(rof_check_grid(d));
+    if (rof_strip_applies(d) && rof_tb2d_depth(d, iters) == 0 && !rof_persist2d_applies(d, iters))
+        return rof_strip_run(f, u_out, lam_arr, lam, iters, tau, epsil, d, s, info, u_init);
     Scratch scratch(s);
     const long long nparts = rof_partial_slots(d);
     IterControl ctl(s, scratch, iters, epsil, nparts);

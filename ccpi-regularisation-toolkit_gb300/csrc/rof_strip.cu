@@ -1,0 +1,186 @@
+// ROF-TV on 2D images, several iterations per launch (strip2d.cuh).
+//
+// The arithmetic is k_rof_pair2d's, operation by operation (ROF_TV_core.c:
+// 102-160).  An iteration of a strip needs one row of U above and below it;
+// the y flux D1 of the row above is recomputed from that row.
+#include "drivers.cuh"
+#include "nvtx.cuh"
+#include "rof_tiled.cuh"
+#include "strip2d.cuh"
+
+namespace cilreg {
+
+namespace {
+
+using namespace strip;
+
+__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
+    const float2 m = make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
+                                 fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
+    return mul2(m, m);
+}
+
+// 1/sqrt(s) for s >= 1e-8: normal, so the flush-to-zero form of the same
+// approximation needs none of the scaling that subnormal arguments do
+__device__ __forceinline__ float rsqrt_normal(float s) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+    return r;
+}
+// ONCE: the result is only used by one subtraction
+template <bool ONCE = false>
+__device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
+    const float2 r = make_float2(rsqrt_normal(s.x), rsqrt_normal(s.y));
+    return ONCE ? mul2_rn(dp, r) : mul2(dp, r);
+}
+
+template <int R, bool CHECK, bool LARR>
+__global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
+    k_rof_strip2d(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F,
+                  const float* __restrict__ lam_arr, float lam, float tau, int nx, int ny, int margin, int count,
+                  bool aligned, const StopCtl* ctl, double2* partials) {
+    __shared__ float2 first[2][NW][32], last[2][NW][32];
+    const Place<R> q(nx, ny, margin, aligned);
+    const int lane = q.lane, w = q.w, Y = q.Y;
+    // f and the lambda map never change during a run: loaded before waiting
+    // for the previous launch (launch_pdl)
+    float2 f[R], l[LARR ? R : 1], u[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        f[r] = q.load_const(F, r);
+        if (LARR) l[r] = q.load_const(lam_arr, r);
+    }
+    if (!LARR) l[0] = splat(lam);
+    pdl_wait();
+    pdl_trigger();
+    if (ctl->stop) return;
+#pragma unroll
+    for (int r = 0; r < R; r++) u[r] = q.load(U, r);
+    const float2 EPS2 = splat(1.0e-8f), tau2 = splat(tau);
+    float2 pa = splat(0.f), pb = splat(0.f);
+
+    // above: the row over the strip (the mirrored row 1 over row 0), next: the
+    // row under that one
+    auto iterate = [&](auto edge_, float2 above, float2 next, float2 below, bool sum) {
+        constexpr bool EDGE = decltype(edge_)::value;
+        // squared minmod of the x differences of a row, and its forward difference
+        auto along_x = [&](float2& c, float2& xp, float2& mx2) {
+            float lo = left_of(c), hi = right_of(c);
+            if (EDGE) {
+                if (q.odd_end) c.y = lo;  // the mirrored pixel beyond an odd row
+                if (q.at_left) lo = c.y;
+                if (q.at_right) hi = c.x;
+            }
+            const float dxc = c.y - c.x;
+            xp = make_float2(dxc, hi - c.y);
+            mx2 = minmod_sq2(xp, make_float2(c.x - lo, dxc));
+        };
+        float2 d1l;  // D1 of the row above
+        {
+            float2 c = above, xp, mx2;
+            along_x(c, xp, mx2);
+            const float2 yp = sub2(next, c);
+            d1l = normalise2(yp, add2(fma2(yp, yp, mx2), EPS2));
+        }
+        float2 ym = sub2(u[0], above);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            float2 c = u[r], xp, mx2;
+            const float2 dn = (r < R - 1) ? u[r + 1 < R ? r + 1 : r] : below;
+            float2 yp = sub2(dn, c);
+            if (EDGE && r == q.bottom) yp = neg2(ym);  // mirrored: the row above is also the row below
+            along_x(c, xp, mx2);
+            const float2 my2 = minmod_sq2(yp, ym);
+            const float2 s1 = add2(fma2(yp, yp, mx2), EPS2);
+            const float2 d1 = (r == R - 1) ? normalise2<true>(yp, s1) : normalise2(yp, s1);
+            const float2 d2 = normalise2(xp, add2(fma2(xp, xp, my2), EPS2));
+            float d2l = left_of(d2);
+            if (EDGE && q.at_left) d2l = d2.y;
+            const float2 div = add2(sub2(d1, d1l), sub2(d2, make_float2(d2l, d2.x)));
+            const float2 t = sub2(c, f[r]);
+            const float2 un = fma2(tau2, fma2(l[LARR ? r : 0], div, neg2(t)), c);
+            if (CHECK && sum && Y + r >= q.y0 && Y + r < q.y1) {
+                const float2 df = sub2(un, c);
+                const float2 dm = make_float2(q.vx ? df.x : 0.f, q.vy ? df.y : 0.f);
+                const float2 um = make_float2(q.vx ? un.x : 0.f, q.vy ? un.y : 0.f);
+                pa = fma2(dm, dm, pa);
+                pb = fma2(um, um, pb);
+            }
+            u[r] = un;
+            ym = yp;
+            d1l = d1;
+        }
+    };
+    for (int t = 0; t < count; t++) {
+        const int b = t & 1;
+        first[b][w][lane] = u[0];
+        last[b][w][lane] = u[R - 1];
+        __syncthreads();
+        const float2 below = w < NW - 1 ? first[b][w + 1][lane] : u[R - 1];
+        const float2 above = Y == 0 ? u[1] : (w > 0 ? last[b][w - 1][lane] : u[0]);
+        const float2 next = Y == 0 ? (R > 2 ? u[R > 2 ? 2 : 0] : below) : u[0];
+        if (q.edge)
+            iterate(std::true_type{}, above, ny == 2 && Y == 0 ? u[0] : next, below, t == count - 1);
+        else
+            iterate(std::false_type{}, above, next, below, t == count - 1);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
+    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+}
+
+using Kernel = decltype(&k_rof_strip2d<2, false, false>);
+template <int R>
+Kernel pick_r(bool check, bool larr) {
+    return check ? (larr ? k_rof_strip2d<R, true, true> : k_rof_strip2d<R, true, false>)
+                 : (larr ? k_rof_strip2d<R, false, true> : k_rof_strip2d<R, false, false>);
+}
+Kernel pick(int R, bool check, bool larr) {
+    return R == 2 ? pick_r<2>(check, larr) : R == 3 ? pick_r<3>(check, larr)
+         : R == 4 ? pick_r<4>(check, larr) : pick_r<6>(check, larr);
+}
+
+}  // namespace
+
+bool rof_strip_applies(const Dims& d) {
+    const char* ek = getenv("CILREG_ROF_KERNEL");
+    return d.nz == 1 && d.nx > 1 && d.ny > 1 && d.n < (1LL << 31) && !(ek && ek[0] != '\0') && strip::enabled();
+}
+
+int rof_strip_run(const float* f, float* u_out, const float* lam_arr, float lam, int iters, float tau, float epsil,
+                  const Dims& d, cudaStream_t s, float* info, const float* u_init) {
+    static const Choices choices = {1, 4, {2, 3, 4, 6}, {2, 2, 2, 1}, 660.0, 300.0};
+    const bool checking = epsil != 0.0f;
+    const Plan P = plan(d.nx, d.ny, iters, checking, choices);
+    Scratch scratch(s);
+    IterControl ctl(s, scratch, iters, epsil, P.nblocks);
+    CILREG_TRY(ctl.status());
+    const float* start = u_init ? u_init : f;
+    const size_t bytes = sizeof(float) * (size_t)d.n;
+    if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, start, bytes, cudaMemcpyDeviceToDevice, s));
+    // launch k writes bufs[(nl - 1 - k) & 1], so that the last one writes u_out
+    const int nl = count_spans(iters, P.T, checking);
+    float* alt = nl > 1 ? scratch.floats(d.n) : nullptr;
+    if (nl > 1 && !alt) return scratch.status();
+    float* bufs[2] = {u_out, alt};
+    const bool larr = lam_arr != nullptr;
+    const bool aligned = host_aligned8(start) && host_aligned8(u_out) && host_aligned8(f) &&
+                         (!larr || host_aligned8(lam_arr));
+    CILREG_TRY(for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
+        const float* src = k == 0 ? start : bufs[(nl - k) & 1];
+        CILREG_CUDA(launch_pdl(pick(P.R, sp.check, larr), P.grid, dim3(32, NW, 1), 0, s, src, bufs[(nl - 1 - k) & 1], f,
+                               lam_arr, lam, tau, d.nx, d.ny, P.margin, sp.count, aligned,
+                               (const StopCtl*)ctl.ctl(), ctl.partials()));
+        note_launch();
+        if (!sp.check) return 0;
+        CILREG_TRY(ctl.after_check(sp.first + sp.count - 1, P.nblocks));
+        return ctl.host_should_stop() ? 1 : 0;
+    }));
+    StopCtl done;
+    CILREG_TRY(ctl.finish(info, &done));
+    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
+        CILREG_CUDA(cudaMemcpyAsync(u_out, alt, bytes, cudaMemcpyDeviceToDevice, s));
+    return OK;
+}
+
+}  // namespace cilreg

@@ -22,6 +22,12 @@ RofPlan rof_pair_plan(const Dims& d);
 int rof_pair_step(const RofPlan& T, const float* cur, float* nxt, const float* f, const float* lam_arr, float lam,
                   float tau, const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s);
 
+// 2D images of fewer than 2^31 pixels run several iterations per launch
+// (rof_strip.cu; CILREG_ROF_KERNEL or CILREG_STRIP2D=0 keep one per launch)
+bool rof_strip_applies(const Dims& d);
+int rof_strip_run(const float* f, float* u_out, const float* lam_arr, float lam, int iters, float tau, float epsil,
+                  const Dims& d, cudaStream_t s, float* info, const float* u_init);
+
 // one iteration: reads cur, writes nxt; on a check iteration one FP64 partial
 // per CTA (RofPlan::nblocks of them)
 int rof_tiled_step(const RofPlan& T, const float* cur, float* nxt, const float* f, const float* lam_arr, float lam,

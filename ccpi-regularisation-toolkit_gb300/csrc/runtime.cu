@@ -1,5 +1,6 @@
 // Host runtime: errors, devices, per-thread streams, scratch, stopping control.
 #include "runtime.cuh"
+#include "strip2d.cuh"
 
 #include <stdarg.h>
 #include <stdlib.h>
@@ -122,6 +123,20 @@ int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chu
     }
     return best;
 }
+
+namespace strip {
+
+bool enabled() {
+    const char* e = getenv("CILREG_STRIP2D");
+    return !(e && e[0] == '0' && e[1] == '\0');
+}
+
+bool forced(int* R, int* T) {
+    const char* e = getenv("CILREG_STRIP2D");
+    return e && sscanf(e, "%d,%d", R, T) == 2;
+}
+
+}  // namespace strip
 
 // ---------------------------------------------------------------------------
 Scratch::~Scratch() {

@@ -1,0 +1,216 @@
+// 2D images, several iterations per launch: the tile scheme shared by the
+// strip kernels.
+//
+// What bounds a 2D iteration launched by itself is not its bytes or its
+// arithmetic but the launch: a 512^2 image's iteration takes 0.1-0.3 us of
+// the chip's issue slots and 2.4-4 us as a graph node.  A strip kernel loads
+// a tile with a halo of `margin` pixels once, runs `count` <= margin
+// iterations on it and stores the part that no cut side has reached.
+//
+// A CTA of NW warps holds a tile of 64 x (NW R) pixels entirely in registers:
+// a lane holds a pixel pair (x, x+1) of R consecutive rows, a warp whole rows
+// of 64 pixels.  Then
+//   * the x neighbours of a pair are its own other pixel and one shuffle;
+//   * the y neighbours are the thread's own registers, except at the first
+//     and last row of a strip, which every warp publishes in shared memory
+//     (two slots, so one barrier per iteration suffices);
+//   * what an iteration needs of a row above or below the strip (a flux, a
+//     projected dual) is recomputed from the published row instead of being
+//     exchanged after a second barrier.
+// Pixels within t of a cut side of the tile are stale after t iterations;
+// sides on the image's edge are exact (the mirrored neighbour, by selects
+// that only strips at the edge execute), so the first and last tile of an
+// axis have no halo on that side.
+#pragma once
+
+#include "pair.cuh"
+
+namespace cilreg {
+namespace strip {
+
+using namespace pair;
+
+constexpr int NW = 16;       // warps of a CTA
+constexpr int NT = 32 * NW;  // threads of a CTA
+constexpr int SW = 64;       // tile width
+constexpr int MAXT = 16;     // largest number of iterations per launch
+
+struct Plan {
+    int R = 0;       // rows per thread; 0: the image does not run strips
+    int T = 0;       // most iterations per launch
+    int margin = 0;  // halo of the tiles
+    dim3 grid;
+    long long nblocks = 0;
+};
+
+// CILREG_STRIP2D=0 runs 2D images one iteration per launch; =R,T asks for R
+// rows per thread and T iterations per launch where they are among the choices
+// (A/B checks and tests)
+bool enabled();
+bool forced(int* R, int* T);
+
+// tiles that cover n pixels: tile i starts at i (len - 2 margin), the first
+// and the last reach the image's edges
+inline int tiles(int n, int len, int margin) {
+    const int step = len - 2 * margin;
+    return n <= len ? 1 : 1 + (n - len + step - 1) / step;
+}
+
+// The rows per thread and the iterations per launch (1 .. 16; 5 with a
+// stopping rule, whose checks end a launch) with the lowest modelled time per
+// iteration, in cycles.  A launch costs LAUNCH and then its waves of CTAs; a
+// wave costs START (a tile's loads and stores) and lat + R lat_row per
+// iteration (the dependent instructions of a warp's rows) with one CTA per SM,
+// PAIRED times that with two (STEADY where CTAs replace each other as they
+// end).  Fitted to ROF on images of 181x217 to 3000x2900 (within 15%); the
+// other regularisers bring their own lat and lat_row.
+struct Choices {
+    int radius;       // stale pixels per iteration at a cut side
+    int n;            // number of kernels
+    int rows[4];      // their rows per thread
+    int resident[4];  // CTAs per SM (1 or 2)
+    double lat, lat_row;
+};
+constexpr double LAUNCH = 1500.0, START = 2200.0, PAIRED = 1.65, STEADY = 1.4;
+inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
+    int fr = 0, ft = 0;
+    const bool ask = forced(&fr, &ft);
+    for (int pass = ask ? 0 : 1; pass < 2; pass++) {
+        Plan best;
+        double best_cost = 0.0;
+        const int tmax = checking ? 5 : (iters < 1 ? 1 : (iters < MAXT ? iters : MAXT));
+        for (int q = 0; q < c.n; q++) {
+            const int R = c.rows[q], H = NW * R;
+            if (pass == 0 && R != fr) continue;
+            for (int t = checking ? 5 : 1; t <= tmax; t++) {
+                const int m = t * c.radius;
+                if (2 * m > SW / 2 || 2 * m > H - 14) break;  // tiles keep half their width and 14 rows
+                if (pass == 0 && !checking && t != (ft < tmax ? ft : tmax)) continue;
+                const long long nb = (long long)tiles(nx, SW, m) * tiles(ny, H, m);
+                const double per_sm = (double)nb / sm_count();
+                const int res = c.resident[q];
+                const double one = START + t * (c.lat + R * c.lat_row), two = one * (res == 2 ? PAIRED : 1.0);
+                double wait;
+                if (per_sm <= 1.0)
+                    wait = one;
+                else if (per_sm <= 2.0 * res)
+                    wait = per_sm <= res ? two : (per_sm <= 3.0 && res == 2 ? one + two : 2.0 * two);
+                else
+                    wait = (per_sm / res + 0.3) * one * (res == 2 ? STEADY : 1.0);
+                const double cost = (LAUNCH + wait) / t;
+                if (best.R == 0 || cost < best_cost) {
+                    best_cost = cost;
+                    best.R = R;
+                    best.T = t;
+                    best.margin = m;
+                    best.grid = dim3((unsigned)tiles(nx, SW, m), (unsigned)tiles(ny, H, m), 1);
+                    best.nblocks = nb;
+                }
+            }
+        }
+        if (best.R) return best;
+    }
+    return Plan{};
+}
+
+// a thread's place in its tile and what it may store
+template <int R>
+struct Place {
+    int lane, w;
+    int X, Y;        // pixel of the thread's first voxel
+    int nx, ny;
+    bool vx, vy;     // columns X, X+1 are stored
+    int y0, y1;      // rows [y0, y1) are stored
+    bool edge;       // an end of the rows or the last row lies in the strip (uniform over the warp)
+    bool at_left, at_right, odd_end;  // the pair starts a row; ends it; its first pixel ends it
+    int bottom;      // the strip's row that is the image's last, if any
+    int c0, c1;      // columns clamped into the image
+    bool vec;        // 8-byte accesses
+    __device__ __forceinline__ Place(int nx_, int ny_, int margin, bool aligned) : nx(nx_), ny(ny_) {
+        constexpr int H = NW * R;
+        lane = threadIdx.x;
+        w = threadIdx.y;
+        const int X0 = blockIdx.x * (SW - 2 * margin), Y0 = blockIdx.y * (H - 2 * margin);
+        X = X0 + 2 * lane;
+        Y = Y0 + w * R;
+        const int xa = X0 ? X0 + margin : 0, xb = (X0 + SW >= nx) ? nx : X0 + SW - margin;
+        y0 = Y0 ? Y0 + margin : 0;
+        y1 = (Y0 + H >= ny) ? ny : Y0 + H - margin;
+        vx = X >= xa && X < xb;
+        vy = X + 1 >= xa && X + 1 < xb;
+        edge = X0 == 0 || X0 + SW >= nx || (Y < ny && Y + R >= ny);
+        at_left = X == 0;
+        at_right = X + 2 == nx;
+        odd_end = X + 1 == nx;
+        bottom = ny - 1 - Y;
+        vec = aligned && (nx & 1) == 0;
+        c0 = vec ? min(X, nx - 2) : min(X, nx - 1);
+        c1 = min(X + 1, nx - 1);
+    }
+    __device__ __forceinline__ int row(int r) const { return min(Y + r, ny - 1) * nx; }
+    __device__ __forceinline__ float2 load_const(const float* __restrict__ p, int r) const {
+        const float* q = p + row(r);
+        if (vec) return __ldg(reinterpret_cast<const float2*>(q + c0));
+        return make_float2(__ldg(q + c0), __ldg(q + c1));
+    }
+    __device__ __forceinline__ float2 load(const float* p, int r) const {
+        const float* q = p + row(r);
+        if (vec) return *reinterpret_cast<const float2*>(q + c0);
+        return make_float2(q[c0], q[c1]);
+    }
+    __device__ __forceinline__ void store(float* p, int r, float2 v) const {
+        const int y = Y + r;
+        if (y < y0 || y >= y1) return;
+        float* q = p + (y * nx + X);
+        if (vec && vx && vy) {
+            st2(q, v);
+        } else {
+            if (vx) q[0] = v.x;
+            if (vy) q[1] = v.y;
+        }
+    }
+};
+
+// a * b per component, never merged with a following addition.  A paired
+// product whose only use is a paired addition becomes a fused multiply-add
+// (measured: ROF's last row of a strip differed in the last place from the
+// one-iteration kernel, whose products go through shared memory); two scalar
+// products do not.
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
+    return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+
+// the pixel left of a pair's first and right of its second, from the
+// neighbouring lanes (the tile's outermost lanes get their own pixel back)
+__device__ __forceinline__ float left_of(float2 v) { return __shfl_up_sync(0xffffffffu, v.y, 1); }
+__device__ __forceinline__ float right_of(float2 v) { return __shfl_down_sync(0xffffffffu, v.x, 1); }
+
+// The launches of a run: iterations [first, first + count) each; with a
+// stopping rule every check iteration (0, 5, 10, ...) ends a launch.
+struct Span {
+    int first, count;
+    bool check;
+};
+template <class F>
+int for_spans(int iters, int most, bool checking, F f) {
+    int it = 0, k = 0;
+    while (it < iters) {
+        int n = checking ? (it == 0 ? 1 : 5) : most;
+        if (n > iters - it) n = iters - it;
+        const Span s{it, n, checking && (it + n - 1) % 5 == 0};
+        const int rc = f(k, s);
+        if (rc != 0) return rc < 0 ? rc : 0;
+        it += n;
+        k++;
+    }
+    return 0;
+}
+inline int count_spans(int iters, int most, bool checking) {
+    if (iters <= 0) return 0;
+    return checking ? 1 + (iters - 1 + 4) / 5 : (iters + most - 1) / most;
+}
+// index of the launch that runs check iteration `it`
+inline int span_of_check(int it) { return it / 5; }
+
+}  // namespace strip
+}  // namespace cilreg

@@ -1,0 +1,85 @@
+"""2D images through the strip kernels (several iterations per launch, tiles
+held in registers) against the kernels that run one iteration per launch:
+sizes at the edges of tiles and of strips, odd rows, images of one pixel
+column or row, every choice of rows per thread, and the stopping rule."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (ny, nx): single pixels and rows, one tile, its edges, several tiles
+SHAPES = [(1, 1), (1, 70), (70, 1), (2, 2), (3, 5), (33, 64), (64, 65), (97, 130), (131, 127), (200, 318)]
+PLANS = ["2,1", "2,5", "3,7", "4,5", "4,16", "6,13"]
+
+
+def _calls():
+    from ccpi.filters import regularisersCuPy as R
+
+    return {"rof": lambda f, it, tol, info: R.ROF_TV(f, 0.02, it, 0.001, tolerance_param=tol, infovector=info)}
+
+
+def _image(shape, seed=3):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    y, x = np.mgrid[0 : shape[0], 0 : shape[1]]
+    img = ((x // 9 + y // 7) % 3) * 0.4 + rng.normal(0, 0.05, shape)
+    return torch.from_numpy(img.astype(np.float32)).cuda()
+
+
+def _run(monkeypatch, setting, op, f, it, tol=0.0):
+    monkeypatch.setenv("CILREG_STRIP2D", setting)
+    info = np.zeros(2, np.float32)
+    out = _calls()[op](f, it, tol, info).cpu().numpy()
+    monkeypatch.delenv("CILREG_STRIP2D")
+    return out, info
+
+
+OPS = ["rof"]
+
+
+@pytest.mark.parametrize("op", OPS)
+@pytest.mark.parametrize("shape", SHAPES)
+def test_strips_equal_single_iterations(monkeypatch, op, shape):
+    f = _image(shape)
+    ref, _ = _run(monkeypatch, "0", op, f, 23)
+    tol = 1e-5 * float(np.ptp(ref) or 1.0)
+    for plan in PLANS:
+        out, _ = _run(monkeypatch, plan, op, f, 23)
+        if shape[1] % 2 == 0 and op in BIT_EQUAL:
+            np.testing.assert_array_equal(out, ref, err_msg=plan)
+        else:
+            np.testing.assert_allclose(out, ref, rtol=0, atol=tol, err_msg=plan)
+
+
+# the strip kernel evaluates the one-iteration kernel's expressions (even rows)
+BIT_EQUAL = {"rof"}
+
+
+@pytest.mark.parametrize("op", OPS)
+@pytest.mark.parametrize("shape", [(61, 90), (131, 127)])
+def test_strips_stop_at_the_same_iteration(monkeypatch, op, shape):
+    f = _image(shape)
+    ref, want = _run(monkeypatch, "0", op, f, 203, 2e-3)
+    for plan in ("2,5", "4,5", "1"):
+        out, info = _run(monkeypatch, plan, op, f, 203, 2e-3)
+        assert info[0] == want[0], plan
+        np.testing.assert_allclose(info[1], want[1], rtol=1e-3)
+        np.testing.assert_allclose(out, ref, rtol=0, atol=1e-5 * float(np.ptp(ref)))
+    # the first check, and counts that end between checks
+    for it in (1, 2, 5, 6, 9):
+        ref, _ = _run(monkeypatch, "0", op, f, it, 1e-9)
+        out, _ = _run(monkeypatch, "1", op, f, it, 1e-9)
+        np.testing.assert_allclose(out, ref, rtol=0, atol=1e-5 * float(np.ptp(ref)))
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_strips_take_arrays_off_8_byte_alignment(monkeypatch, op):
+    import torch
+
+    base = torch.zeros(1 + 77 * 130, device="cuda")
+    f = base[1:].view(77, 130)
+    f.copy_(_image((77, 130)))
+    out, _ = _run(monkeypatch, "1", op, f, 17)
+    ref, _ = _run(monkeypatch, "1", op, f.clone(), 17)
+    np.testing.assert_array_equal(out, ref)
