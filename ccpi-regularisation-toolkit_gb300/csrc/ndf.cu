@@ -92,6 +92,8 @@ int ndf_run(const float* f, float* u_out, float lam, float sigma, int iters, flo
     // gives what it gives at 0 up to the sign of a zero flux, and from 0 on a
     // flux whose sign is taken has e != 0 (flux in ndf_tiled.cuh)
     const float sg = fmaxf(sg_ref, 0.0f);
+    if (ndf_strip_applies(d))
+        return ndf_strip_run(pen, f, u_out, lam, sg, isg, iters, tau, epsil, d, s, info, u_init);
     const bool three = d.nz > 1;
     Scratch scratch(s);
     const Launch3 L = plan_launch(d);

@@ -44,36 +44,6 @@ constexpr int AHEAD = 4, RING = 8;
 constexpr int ZCHUNK = 64;
 constexpr size_t SMEM = sizeof(float) * TP * (RING + 4);  // U ring, Fx and Fy (two planes each)
 
-// flux<PEN> (ndf_tiled.cuh) of both components, the products paired
-template <int PEN>
-__device__ __forceinline__ float2 flux2(float2 e, float sg, float2 isg2) {
-    if (PEN == 0) return e;
-    if (PEN == 1) {
-        const float2 r = mul2(e, isg2);
-        return make_float2((fabsf(e.x) > sg) ? copysignf(1.0f, e.x) : r.x,
-                           (fabsf(e.y) > sg) ? copysignf(1.0f, e.y) : r.y);
-    }
-    if (PEN == 2) {
-        const float2 r = mul2(e, isg2);
-        const float2 q = fma2(r, r, splat(1.0f));
-        return mul2(e, make_float2(__frcp_rn(q.x), __frcp_rn(q.y)));
-    }
-    if (PEN == 3) {
-        const float2 r = mul2(e, isg2);
-        const float2 w = fma2(neg2(r), r, splat(1.0f));
-        const float2 v = mul2(e, mul2(w, w));
-        return make_float2((fabsf(e.x) <= sg) ? v.x : 0.0f, (fabsf(e.y) <= sg) ? v.y : 0.0f);
-    }
-    if (PEN == 4) return make_float2((fabsf(e.x) > sg) ? 0.0f : e.x, (fabsf(e.y) > sg) ? 0.0f : e.y);
-    // PEN == 5
-    const float2 r = mul2(e, isg2);
-    auto one = [&](float ev, float rv) {
-        if (fabsf(ev) <= 2.0f * sg) return (fabsf(ev) > sg) ? copysignf(1.0f, ev) : rv;
-        return 0.0f;
-    };
-    return make_float2(one(e.x, r.x), one(e.y, r.y));
-}
-
 template <int PEN, bool CHECK, bool ALIGNED>
 __global__ void __launch_bounds__(NTP, 4)
     k_ndf_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam, float sg,

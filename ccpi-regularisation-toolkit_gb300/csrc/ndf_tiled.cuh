@@ -3,6 +3,7 @@
 // streaming kernel's entry points.
 #pragma once
 
+#include "pair.cuh"
 #include "runtime.cuh"
 
 namespace cilreg {
@@ -38,6 +39,37 @@ __device__ __forceinline__ float flux(float e, float sg, float isg) {
 // only through e itself or its sign copy), so the flux through a face can be formed
 // once and used with opposite signs by the two voxels that share it.
 
+// flux<PEN> of both components, the products paired
+template <int PEN>
+__device__ __forceinline__ float2 flux2(float2 e, float sg, float2 isg2) {
+    if (PEN == 0) return e;
+    if (PEN == 1) {
+        const float2 r = pair::mul2(e, isg2);
+        return make_float2((fabsf(e.x) > sg) ? copysignf(1.0f, e.x) : r.x,
+                           (fabsf(e.y) > sg) ? copysignf(1.0f, e.y) : r.y);
+    }
+    if (PEN == 2) {
+        const float2 r = pair::mul2(e, isg2);
+        const float2 q = pair::fma2(r, r, pair::splat(1.0f));
+        // scalar products: a paired one may merge with the addition that takes it
+        return make_float2(__fmul_rn(e.x, __frcp_rn(q.x)), __fmul_rn(e.y, __frcp_rn(q.y)));
+    }
+    if (PEN == 3) {
+        const float2 r = pair::mul2(e, isg2);
+        const float2 w = pair::fma2(pair::neg2(r), r, pair::splat(1.0f));
+        const float2 v = pair::mul2(e, pair::mul2(w, w));
+        return make_float2((fabsf(e.x) <= sg) ? v.x : 0.0f, (fabsf(e.y) <= sg) ? v.y : 0.0f);
+    }
+    if (PEN == 4) return make_float2((fabsf(e.x) > sg) ? 0.0f : e.x, (fabsf(e.y) > sg) ? 0.0f : e.y);
+    // PEN == 5
+    const float2 r = pair::mul2(e, isg2);
+    auto one = [&](float ev, float rv) {
+        if (fabsf(ev) <= 2.0f * sg) return (fabsf(ev) > sg) ? copysignf(1.0f, ev) : rv;
+        return 0.0f;
+    };
+    return make_float2(one(e.x, r.x), one(e.y, r.y));
+}
+
 struct NdfPlan {
     dim3 grid, block;
     long long nblocks = 0;
@@ -45,6 +77,13 @@ struct NdfPlan {
     bool use = false;   // false: the per-voxel kernel of ndf.cu runs instead
     bool pair = false;  // the two-voxels-per-thread kernel (ndf_pair.cu)
 };
+
+// 2D images run several iterations per launch (ndf_strip.cu;
+// CILREG_NDF_KERNEL or CILREG_STRIP2D=0 keep one per launch); sg and isg as
+// the kernels take them
+bool ndf_strip_applies(const Dims& d);
+int ndf_strip_run(int pen, const float* f, float* u_out, float lam, float sg, float isg, int iters, float tau,
+                  float epsil, const Dims& d, cudaStream_t s, float* info, const float* u_init);
 
 // the plan of the kernel that runs for `d`: volumes and images with nx even
 // and fewer than 2^31 voxels run k_ndf_pair (3D) or k_ndf_pair2d, others

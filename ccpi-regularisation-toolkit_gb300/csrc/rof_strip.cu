@@ -65,12 +65,8 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         constexpr bool EDGE = decltype(edge_)::value;
         // squared minmod of the x differences of a row, and its forward difference
         auto along_x = [&](float2& c, float2& xp, float2& mx2) {
-            float lo = left_of(c), hi = right_of(c);
-            if (EDGE) {
-                if (q.odd_end) c.y = lo;  // the mirrored pixel beyond an odd row
-                if (q.at_left) lo = c.y;
-                if (q.at_right) hi = c.x;
-            }
+            float lo, hi;
+            x_neighbours<EDGE>(q, c, lo, hi);
             const float dxc = c.y - c.x;
             xp = make_float2(dxc, hi - c.y);
             mx2 = minmod_sq2(xp, make_float2(c.x - lo, dxc));
@@ -99,13 +95,7 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
             const float2 div = add2(sub2(d1, d1l), sub2(d2, make_float2(d2l, d2.x)));
             const float2 t = sub2(c, f[r]);
             const float2 un = fma2(tau2, fma2(l[LARR ? r : 0], div, neg2(t)), c);
-            if (CHECK && sum && Y + r >= q.y0 && Y + r < q.y1) {
-                const float2 df = sub2(un, c);
-                const float2 dm = make_float2(q.vx ? df.x : 0.f, q.vy ? df.y : 0.f);
-                const float2 um = make_float2(q.vx ? un.x : 0.f, q.vy ? un.y : 0.f);
-                pa = fma2(dm, dm, pa);
-                pb = fma2(um, um, pb);
-            }
+            if (CHECK && sum) add_norms(q, r, un, c, pa, pb);
             u[r] = un;
             ym = yp;
             d1l = d1;
@@ -135,52 +125,28 @@ Kernel pick_r(bool check, bool larr) {
     return check ? (larr ? k_rof_strip2d<R, true, true> : k_rof_strip2d<R, true, false>)
                  : (larr ? k_rof_strip2d<R, false, true> : k_rof_strip2d<R, false, false>);
 }
-Kernel pick(int R, bool check, bool larr) {
-    return R == 2 ? pick_r<2>(check, larr) : R == 3 ? pick_r<3>(check, larr)
-         : R == 4 ? pick_r<4>(check, larr) : pick_r<6>(check, larr);
+Kernel pick(const Plan& P, bool check, bool larr) {
+    return P.R == 2 ? pick_r<2>(check, larr) : P.R == 3 ? pick_r<3>(check, larr)
+         : P.R == 4 ? pick_r<4>(check, larr) : pick_r<6>(check, larr);
 }
 
 }  // namespace
 
 bool rof_strip_applies(const Dims& d) {
     const char* ek = getenv("CILREG_ROF_KERNEL");
-    return d.nz == 1 && d.nx > 1 && d.ny > 1 && d.n < (1LL << 31) && !(ek && ek[0] != '\0') && strip::enabled();
+    return strip::applies(d) && !(ek && ek[0] != '\0');
 }
 
 int rof_strip_run(const float* f, float* u_out, const float* lam_arr, float lam, int iters, float tau, float epsil,
                   const Dims& d, cudaStream_t s, float* info, const float* u_init) {
     static const Choices choices = {1, 4, {2, 3, 4, 6}, {2, 2, 2, 1}, 660.0, 300.0};
-    const bool checking = epsil != 0.0f;
-    const Plan P = plan(d.nx, d.ny, iters, checking, choices);
-    Scratch scratch(s);
-    IterControl ctl(s, scratch, iters, epsil, P.nblocks);
-    CILREG_TRY(ctl.status());
-    const float* start = u_init ? u_init : f;
-    const size_t bytes = sizeof(float) * (size_t)d.n;
-    if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, start, bytes, cudaMemcpyDeviceToDevice, s));
-    // launch k writes bufs[(nl - 1 - k) & 1], so that the last one writes u_out
-    const int nl = count_spans(iters, P.T, checking);
-    float* alt = nl > 1 ? scratch.floats(d.n) : nullptr;
-    if (nl > 1 && !alt) return scratch.status();
-    float* bufs[2] = {u_out, alt};
     const bool larr = lam_arr != nullptr;
-    const bool aligned = host_aligned8(start) && host_aligned8(u_out) && host_aligned8(f) &&
-                         (!larr || host_aligned8(lam_arr));
-    CILREG_TRY(for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
-        const float* src = k == 0 ? start : bufs[(nl - k) & 1];
-        CILREG_CUDA(launch_pdl(pick(P.R, sp.check, larr), P.grid, dim3(32, NW, 1), 0, s, src, bufs[(nl - 1 - k) & 1], f,
-                               lam_arr, lam, tau, d.nx, d.ny, P.margin, sp.count, aligned,
-                               (const StopCtl*)ctl.ctl(), ctl.partials()));
-        note_launch();
-        if (!sp.check) return 0;
-        CILREG_TRY(ctl.after_check(sp.first + sp.count - 1, P.nblocks));
-        return ctl.host_should_stop() ? 1 : 0;
-    }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
-        CILREG_CUDA(cudaMemcpyAsync(u_out, alt, bytes, cudaMemcpyDeviceToDevice, s));
-    return OK;
+    return run_flow(choices, f, u_init ? u_init : f, u_out, iters, epsil, d, s, info, !larr || host_aligned8(lam_arr),
+                    [&](const Plan& P, const Span& sp, const float* src, float* dst, bool aligned, IterControl& ctl) {
+                        return launch_pdl(pick(P, sp.check, larr), P.grid, dim3(32, NW, 1), 0, s, src, dst, f, lam_arr,
+                                          lam, tau, d.nx, d.ny, P.margin, sp.count, aligned,
+                                          (const StopCtl*)ctl.ctl(), ctl.partials());
+                    });
 }
 
 }  // namespace cilreg

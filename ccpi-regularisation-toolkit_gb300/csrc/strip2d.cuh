@@ -23,6 +23,7 @@
 // axis have no halo on that side.
 #pragma once
 
+#include "drivers.cuh"
 #include "pair.cuh"
 
 namespace cilreg {
@@ -30,7 +31,7 @@ namespace strip {
 
 using namespace pair;
 
-constexpr int NW = 16;       // warps of a CTA
+constexpr int NW = 16;       // warps of a CTA (32 of 2 rows measured 1.2-1.5 times slower than 16 of 4)
 constexpr int NT = 32 * NW;  // threads of a CTA
 constexpr int SW = 64;       // tile width
 constexpr int MAXT = 16;     // largest number of iterations per launch
@@ -89,7 +90,8 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
                 const long long nb = (long long)tiles(nx, SW, m) * tiles(ny, H, m);
                 const double per_sm = (double)nb / sm_count();
                 const int res = c.resident[q];
-                const double one = START + t * (c.lat + R * c.lat_row), two = one * (res == 2 ? PAIRED : 1.0);
+                const double one = START + t * (c.lat + R * c.lat_row);
+                const double two = one * (res == 2 ? PAIRED : 1.0);
                 double wait;
                 if (per_sm <= 1.0)
                     wait = one;
@@ -121,7 +123,7 @@ struct Place {
     int nx, ny;
     bool vx, vy;     // columns X, X+1 are stored
     int y0, y1;      // rows [y0, y1) are stored
-    bool edge;       // an end of the rows or the last row lies in the strip (uniform over the warp)
+    bool edge;       // an end of the rows, or the last row, lies in the strip or right under it (uniform over the warp)
     bool at_left, at_right, odd_end;  // the pair starts a row; ends it; its first pixel ends it
     int bottom;      // the strip's row that is the image's last, if any
     int c0, c1;      // columns clamped into the image
@@ -138,7 +140,7 @@ struct Place {
         y1 = (Y0 + H >= ny) ? ny : Y0 + H - margin;
         vx = X >= xa && X < xb;
         vy = X + 1 >= xa && X + 1 < xb;
-        edge = X0 == 0 || X0 + SW >= nx || (Y < ny && Y + R >= ny);
+        edge = X0 == 0 || X0 + SW >= nx || (Y < ny && Y + R + 1 >= ny);
         at_left = X == 0;
         at_right = X + 2 == nx;
         odd_end = X + 1 == nx;
@@ -211,6 +213,67 @@ inline int count_spans(int iters, int most, bool checking) {
 }
 // index of the launch that runs check iteration `it`
 inline int span_of_check(int it) { return it / 5; }
+
+// the images that strips take
+inline bool applies(const Dims& d) { return d.nz == 1 && d.nx > 1 && d.ny > 1 && d.n < (1LL << 31) && enabled(); }
+
+// an x neighbour pair of v: (x-1, x) and (x+1, x+2), mirrored at the ends of
+// the image's rows; the pixel beyond an odd row takes its mirrored value
+template <bool EDGE, int R>
+__device__ __forceinline__ void x_neighbours(const Place<R>& q, float2& v, float& lo, float& hi) {
+    lo = left_of(v);
+    hi = right_of(v);
+    if (EDGE) {
+        if (q.odd_end) v.y = lo;
+        if (q.at_left) lo = v.y;
+        if (q.at_right) hi = v.x;
+    }
+}
+
+// adds the stored pixels' squared change and square of one row
+template <int R>
+__device__ __forceinline__ void add_norms(const Place<R>& q, int r, float2 un, float2 u, float2& pa, float2& pb) {
+    if (q.Y + r < q.y0 || q.Y + r >= q.y1) return;
+    const float2 df = sub2(un, u);
+    const float2 dm = make_float2(q.vx ? df.x : 0.f, q.vy ? df.y : 0.f);
+    const float2 um = make_float2(q.vx ? un.x : 0.f, q.vy ? un.y : 0.f);
+    pa = fma2(dm, dm, pa);
+    pb = fma2(um, um, pb);
+}
+
+// The run of a regulariser whose state is one image U beside f (ROF, NDF,
+// Diff4th, LLT-ROF): launch(plan, span, src, dst, aligned, ctl) enqueues one
+// launch.  Launch k writes bufs[(nl - 1 - k) & 1], so the last writes u_out;
+// a run that stops early on the other buffer copies it.
+template <class Launch>
+int run_flow(const Choices& choices, const float* f, const float* start, float* u_out, int iters, float epsil,
+             const Dims& d, cudaStream_t s, float* info, bool aligned, Launch launch) {
+    const bool checking = epsil != 0.0f;
+    const Plan P = plan(d.nx, d.ny, iters, checking, choices);
+    Scratch scratch(s);
+    IterControl ctl(s, scratch, iters, epsil, P.nblocks);
+    CILREG_TRY(ctl.status());
+    const size_t bytes = sizeof(float) * (size_t)d.n;
+    if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, start, bytes, cudaMemcpyDeviceToDevice, s));
+    const int nl = count_spans(iters, P.T, checking);
+    float* alt = nl > 1 ? scratch.floats(d.n) : nullptr;
+    if (nl > 1 && !alt) return scratch.status();
+    float* bufs[2] = {u_out, alt};
+    aligned = aligned && host_aligned8(f) && host_aligned8(start) && host_aligned8(u_out);
+    CILREG_TRY(for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
+        const float* src = k == 0 ? start : bufs[(nl - k) & 1];
+        CILREG_CUDA(launch(P, sp, src, bufs[(nl - 1 - k) & 1], aligned, ctl));
+        note_launch();
+        if (!sp.check) return 0;
+        CILREG_TRY(ctl.after_check(sp.first + sp.count - 1, P.nblocks));
+        return ctl.host_should_stop() ? 1 : 0;
+    }));
+    StopCtl done;
+    CILREG_TRY(ctl.finish(info, &done));
+    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
+        CILREG_CUDA(cudaMemcpyAsync(u_out, alt, bytes, cudaMemcpyDeviceToDevice, s));
+    return OK;
+}
 
 }  // namespace strip
 }  // namespace cilreg

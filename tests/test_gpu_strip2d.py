@@ -15,7 +15,13 @@ PLANS = ["2,1", "2,5", "3,7", "4,5", "4,16", "6,13"]
 def _calls():
     from ccpi.filters import regularisersCuPy as R
 
-    return {"rof": lambda f, it, tol, info: R.ROF_TV(f, 0.02, it, 0.001, tolerance_param=tol, infovector=info)}
+    calls = {"rof": lambda f, it, tol, info: R.ROF_TV(f, 0.02, it, 0.001, tolerance_param=tol, infovector=info),
+             "d4": lambda f, it, tol, info: R.Diff4th(f, 0.8, 0.02, it, 1e-4, tol, infovector=info),
+             "llt": lambda f, it, tol, info: R.LLT_ROF(f, 0.02, 0.01, it, 1e-3, tol, infovector=info)}
+    for p in range(6):  # 0: linear diffusion
+        calls[f"ndf{p}"] = lambda f, it, tol, info, p=p: R.NDF(f, 0.02, 0.05 * (p > 0), it, 0.01, max(p, 1), tol,
+                                                               infovector=info)
+    return calls
 
 
 def _image(shape, seed=3):
@@ -35,7 +41,7 @@ def _run(monkeypatch, setting, op, f, it, tol=0.0):
     return out, info
 
 
-OPS = ["rof"]
+OPS = ["rof", "d4", "llt"] + [f"ndf{p}" for p in range(6)]
 
 
 @pytest.mark.parametrize("op", OPS)
@@ -53,7 +59,7 @@ def test_strips_equal_single_iterations(monkeypatch, op, shape):
 
 
 # the strip kernel evaluates the one-iteration kernel's expressions (even rows)
-BIT_EQUAL = {"rof"}
+BIT_EQUAL = set(OPS)
 
 
 @pytest.mark.parametrize("op", OPS)
