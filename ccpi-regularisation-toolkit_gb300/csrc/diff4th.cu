@@ -114,6 +114,9 @@ __global__ void __launch_bounds__(256) k_d4_update(float* __restrict__ U, const 
 int diff4th_run(const float* f, float* u_out, float lam, float sigma, int iters, float tau, float epsil,
                 const Dims& d, cudaStream_t s, float* info) {
     CILREG_RANGE("cilreg Diff4th");
+    const float sg2 = sigma * sigma;  // Diffus4th_order_core.c:51
+    const float isg2 = 1.0f / sg2;    // den / sg2 formed as den * isg2 (within 1 ulp)
+    if (d4_strip_applies(d)) return d4_strip_run(f, u_out, lam, iters, tau, isg2, epsil, d, s, info);
     const bool three = d.nz > 1;
     Scratch scratch(s);
     const Launch3 L = plan_launch(d);
@@ -126,8 +129,6 @@ int diff4th_run(const float* f, float* u_out, float lam, float sigma, int iters,
     float* W = scratch.floats(d.n);
     if (!W) return scratch.status();
     CILREG_CUDA(cudaMemcpyAsync(u_out, f, sizeof(float) * d.n, cudaMemcpyDeviceToDevice, s));
-    const float sg2 = sigma * sigma;  // Diffus4th_order_core.c:51
-    const float isg2 = 1.0f / sg2;    // den / sg2 formed as den * isg2 (within 1 ulp)
     if (stream) {
         // fused iteration, ping-pong between u_out and W's buffer
         float* bufs[2] = {u_out, W};

@@ -20,6 +20,11 @@ bool d4_pair_applies(const Dims& d);
 D4Plan d4_pair_plan(const Dims& d);
 int d4_pair_step(const D4Plan& T, const float* cur, float* nxt, const float* f, float lam, float tau, float isg2,
                  const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s);
+// 2D images run several iterations per launch (diff4th_strip.cu;
+// CILREG_D4_KERNEL or CILREG_STRIP2D=0 keep one per launch)
+bool d4_strip_applies(const Dims& d);
+int d4_strip_run(const float* f, float* u_out, float lam, int iters, float tau, float isg2, float epsil, const Dims& d,
+                 cudaStream_t s, float* info);
 // one iteration: reads cur, writes nxt (distinct buffers); isg2 = 1/sigma^2
 int d4_stream_step(const D4Plan& T, const float* cur, float* nxt, const float* f, float lam, float tau, float isg2,
                    const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s);
