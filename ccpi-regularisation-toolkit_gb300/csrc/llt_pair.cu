@@ -38,35 +38,6 @@ constexpr int NTP = PX * ROWS, TP = TW * ROWS;
 constexpr int OX4 = TW - 4, OY4 = ROWS - 4;
 constexpr int ZCHUNK = 64;
 
-__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
-    const float2 m = make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
-                                 fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
-    return mul2(m, m);
-}
-
-// dp / sqrt(s) per component
-__device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
-    return mul2(dp, make_float2(rsqrtf(s.x), rsqrtf(s.y)));
-}
-
-// v / (|v| + 1e-12), the second difference over its magnitude (llt_term
-// of llt.cu), with the IEEE quotient's value and without its division for
-// almost every v: from |v| = 2^-15 on, 1e-12 is below half an ulp of |v|, so
-// the rounded denominator is |v| and the quotient exactly +-1; v = +-0 gives
-// itself.  Only the other values (below 2^-15, infinite, NaN) divide: a step
-// forms the six terms of its pair by sign copies and, when any of them needs
-// it, all six by the division (one branch).
-__device__ __forceinline__ float llt_sign1(float v) { return (v == 0.0f) ? v : copysignf(1.0f, v); }
-__device__ __forceinline__ float2 llt_sign2(float2 v) { return make_float2(llt_sign1(v.x), llt_sign1(v.y)); }
-__device__ __forceinline__ bool llt_divides(float v) {
-    const float a = fabsf(v);
-    return !(a >= 0x1p-15f && a <= 3.4028234664e38f) && a != 0.0f;
-}
-__device__ __forceinline__ bool llt_divides2(float2 v) { return llt_divides(v.x) | llt_divides(v.y); }
-__device__ __forceinline__ float2 llt_quot2(float2 v) {
-    return make_float2(v.x / (fabsf(v.x) + 1.0e-12f), v.y / (fabsf(v.y) + 1.0e-12f));
-}
-
 template <bool CHECK, bool ALIGNED, int MINB>
 __global__ void __launch_bounds__(NTP, MINB)
     k_llt_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam_rof,
