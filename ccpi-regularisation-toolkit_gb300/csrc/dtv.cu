@@ -68,20 +68,19 @@ int dtv_run(const float* f, const float* ref, float* u_out, float lam, int iters
         const TiledPlan X = fgp_x2_plan(d);
         if (X.use) T = X;
     }
-    IterControl ctl(s, scratch, iters, epsil, T.nblocks);
-    CILREG_TRY(ctl.status());
+    const bool strips = fgp_strip_applies(d);
     float* ring[3][3] = {};
     float* b[3] = {nullptr, nullptr, nullptr};
     for (int c = 0; c < nc; c++) {
         b[c] = scratch.floats(d.n);
         if (!b[c]) return scratch.status();
-        for (int r = 0; r < 3; r++) {
+        for (int r = 0; r < 3 && !strips; r++) {
             ring[r][c] = scratch.floats(d.n);
             if (!ring[r][c]) return scratch.status();
         }
     }
     // P^{-1} = P^{-2} = 0 (calloc'd P, P_prev, R of the reference)
-    for (int r = 1; r < 3; r++)
+    for (int r = 1; r < 3 && !strips; r++)
         for (int c = 0; c < nc; c++) CILREG_CUDA(cudaMemsetAsync(ring[r][c], 0, sizeof(float) * d.n, s));
     {
         const Launch3 L = plan_launch(d);
@@ -101,6 +100,16 @@ int dtv_run(const float* f, const float* ref, float* u_out, float lam, int iters
         cprev = (tk - 1.0f) / tkp1;
         tk = tkp1;
     };
+    if (strips) {
+        std::vector<float> cseq(iters > 0 ? iters : 0);
+        for (float& v : cseq) {
+            v = cprev;
+            advance();
+        }
+        return fgp_strip_run(f, b, u_out, lam, multip, cseq, epsil, nonneg == 1, methodTV != 0, d, s, info, nullptr);
+    }
+    IterControl ctl(s, scratch, iters, epsil, T.nblocks);
+    CILREG_TRY(ctl.status());
     int it = 0;
     constexpr int G = 66;  // replayed block: a multiple of the ring's period 3
     if (!ctl.checking() && d.n <= (1LL << 22) && iters > 2 * G) {

@@ -115,6 +115,19 @@ int fgp_run(const float* f, float* u_out, float lam, int iters, float epsil, int
     CILREG_RANGE("cilreg FGP-TV");
     const bool three = d.nz > 1;
     const int nc = three ? 3 : 2;
+    if (fgp_strip_applies(d)) {
+        // t_{k+1} and the momentum coefficient of every R (FGP_TV_core.c:138-139)
+        std::vector<float> cseq(iters > 0 ? iters : 0);
+        float tk = 1.0f, c = 0.0f;
+        for (float& v : cseq) {
+            v = c;
+            const float tkp1 = (1.0f + sqrtf(1.0f + 4.0f * tk * tk)) * 0.5f;
+            c = (tk - 1.0f) / tkp1;
+            tk = tkp1;
+        }
+        return fgp_strip_run(f, nullptr, u_out, lam, 1.0f / (8.0f * lam), cseq, epsil, nonneg == 1, methodTV != 0, d, s,
+                             info, warm);
+    }
     Scratch scratch(s);
     const Launch3 L = plan_launch(d);
     TiledPlan T = fgp_tiled_plan(d);

@@ -1,6 +1,9 @@
 // Shared-memory tiled FGP-TV iteration (3D), see fgp_tiled.cu.
 #pragma once
 
+#include <vector>
+
+#include "drivers.cuh"
 #include "runtime.cuh"
 
 namespace cilreg {
@@ -124,5 +127,14 @@ bool fgp_x2_batch_usable(const Dims* dims, const float* const* f, float* const* 
 void fgp_x2_tile_grid(const Dims& d, int zc, int& gx, int& gy, int& gz);
 int fgp_x2_batch_step(const FgpBatchVol* d_vols, const int* d_tile_vol, long long ntiles, int it, float c,
                       int nonneg, int aniso, int write_u, int write_p, int check, cudaStream_t s);
+
+// 2D images run several iterations per launch (fgp_strip.cu; CILREG_FGP_KERNEL
+// or CILREG_STRIP2D=0 keep one per launch).  cseq: the momentum coefficient of
+// every iteration; b: FGP-dTV's unit gradient of the reference (two arrays) or
+// null; warm as in fgp_run
+bool fgp_strip_applies(const Dims& d);
+int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam, float multip,
+                  const std::vector<float>& cseq, float epsil, bool nonneg, bool aniso, const Dims& d, cudaStream_t s,
+                  float* info, FgpWarm* warm);
 
 }  // namespace cilreg

@@ -20,13 +20,6 @@ __device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
     return mul2(m, m);
 }
 
-// 1/sqrt(s) for s >= 1e-8: normal, so the flush-to-zero form of the same
-// approximation needs none of the scaling that subnormal arguments do
-__device__ __forceinline__ float rsqrt_normal(float s) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
-    return r;
-}
 // ONCE: the result is only used by one subtraction
 template <bool ONCE = false>
 __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {

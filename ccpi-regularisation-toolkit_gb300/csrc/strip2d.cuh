@@ -60,19 +60,20 @@ inline int tiles(int n, int len, int margin) {
 // The rows per thread and the iterations per launch (1 .. 16; 5 with a
 // stopping rule, whose checks end a launch) with the lowest modelled time per
 // iteration, in cycles.  A launch costs LAUNCH and then its waves of CTAs; a
-// wave costs START (a tile's loads and stores) and lat + R lat_row per
-// iteration (the dependent instructions of a warp's rows) with one CTA per SM,
+// wave costs start + R start_row (a tile's loads and stores) and lat + R
+// lat_row per iteration (a warp's dependent instructions) with one CTA per SM,
 // PAIRED times that with two (STEADY where CTAs replace each other as they
 // end).  Fitted to ROF on images of 181x217 to 3000x2900 (within 15%); the
-// other regularisers bring their own lat and lat_row.
+// other regularisers bring the constants measured on them.
 struct Choices {
     int radius;       // stale pixels per iteration at a cut side
     int n;            // number of kernels
     int rows[4];      // their rows per thread
     int resident[4];  // CTAs per SM (1 or 2)
     double lat, lat_row;
+    double start = 2200.0, start_row = 0.0;
 };
-constexpr double LAUNCH = 1500.0, START = 2200.0, PAIRED = 1.65, STEADY = 1.4;
+constexpr double LAUNCH = 1500.0, PAIRED = 1.65, STEADY = 1.4;
 inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
     int fr = 0, ft = 0;
     const bool ask = forced(&fr, &ft);
@@ -90,7 +91,7 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
                 const long long nb = (long long)tiles(nx, SW, m) * tiles(ny, H, m);
                 const double per_sm = (double)nb / sm_count();
                 const int res = c.resident[q];
-                const double one = START + t * (c.lat + R * c.lat_row);
+                const double one = c.start + R * c.start_row + t * (c.lat + R * c.lat_row);
                 const double two = one * (res == 2 ? PAIRED : 1.0);
                 double wait;
                 if (per_sm <= 1.0)
@@ -180,6 +181,14 @@ struct Place {
 // products do not.
 __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+
+// 1/sqrt(s) for normal s: the flush-to-zero form of rsqrtf's approximation,
+// the same value without the scaling that subnormal arguments need
+__device__ __forceinline__ float rsqrt_normal(float s) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+    return r;
 }
 
 // the pixel left of a pair's first and right of its second, from the
