@@ -96,6 +96,14 @@ private:
     int status_ = 0;
 };
 
+// What the host sees of a run's stopping control: a copy that the finalize
+// kernel of every check writes into page-locked memory, and that check's
+// number, written after it.
+struct StopMirror {
+    StopCtl ctl;
+    int seq;
+};
+
 // Device-resident stopping control for one regulariser run.
 class IterControl {
 public:
@@ -118,9 +126,9 @@ private:
     cudaStream_t stream_;
     StopCtl* d_ctl_ = nullptr;
     double2* d_part_ = nullptr;
-    StopCtl* h_ring_ = nullptr;  // pinned mirror slots
-    cudaEvent_t ev_[4] = {};
-    int nev_ = 0, head_ = 0, pending_ = 0;
+    StopMirror* h_ = nullptr;  // page-locked, written by the device
+    int checks_ = 0;           // checks enqueued
+    int iter_total_;
     float epsil_;
     int status_ = 0;
 };
