@@ -15,10 +15,9 @@ using namespace strip;
 template <int R, bool CHECK>
 __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     k_d4_strip2d(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam, float tau,
-                 float isg2, int nx, int ny, int margin, int count, bool aligned, const StopCtl* ctl,
-                 double2* partials) {
+                 float isg2, Frame fr) {
     __shared__ float2 firstU[NW][32], lastU[NW][32], firstW[NW][32], lastW[NW][32];
-    const Place<R> q(nx, ny, margin, aligned);
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w;
     const float EPS = 1.0e-7f;
     const float2 HALF2 = splat(0.5f), QUART2 = splat(0.25f), TWO2 = splat(2.0f), MTWO2 = splat(-2.0f);
@@ -26,9 +25,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     float2 f[R], u[R];
 #pragma unroll
     for (int r = 0; r < R; r++) f[r] = q.load_const(F, r);  // never changes: loaded before the wait
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->stop) return;
+    if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     float2 pa = splat(0.f), pb = splat(0.f);
@@ -85,7 +82,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
             wm = W[r];
         }
     };
-    for (int t = 0; t < count; t++) {
+    for (int t = 0; t < fr.count; t++) {
         firstU[w][lane] = u[0];
         lastU[w][lane] = u[R - 1];
         __syncthreads();
@@ -101,13 +98,13 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
         const float2 wbelow = w < NW - 1 ? firstW[w + 1][lane] : W[R - 1];
         const float2 wabove = q.Y == 0 ? W[1] : (w > 0 ? lastW[w - 1][lane] : W[0]);
         if (q.edge)
-            update(std::true_type{}, wabove, wbelow, t == count - 1);
+            update(std::true_type{}, wabove, wbelow, t == fr.count - 1);
         else
-            update(std::false_type{}, wabove, wbelow, t == count - 1);
+            update(std::false_type{}, wabove, wbelow, t == fr.count - 1);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_d4_strip2d<2, false>);
@@ -128,10 +125,9 @@ int d4_strip_run(const float* f, float* u_out, float lam, int iters, float tau, 
                  cudaStream_t s, float* info) {
     static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 870.0, 420.0};
     return run_flow(choices, f, f, u_out, iters, epsil, d, s, info, true,
-                    [&](const Plan& P, const Span& sp, const float* src, float* dst, bool aligned, IterControl& ctl) {
-                        return launch_pdl(pick(P, sp.check), P.grid, dim3(32, NW, 1), 0, s, src, dst, f, lam, tau,
-                                          isg2, d.nx, d.ny, P.margin, sp.count, aligned, (const StopCtl*)ctl.ctl(),
-                                          ctl.partials());
+                    [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
+                        return launch_pdl(pick(P, rule), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam, tau,
+                                          isg2, fr);
                     });
 }
 

@@ -27,11 +27,11 @@ struct Args {
     float* qo[2];        // P of the one before; null: not stored
     const float* f;
     const float* b[2];  // FGP-dTV: the reference's unit gradient
-    float* u;           // output, and U_prev of a launch of one check iteration
+    float* u;           // output
+    const float* u_prev;  // of a launch of one check iteration
     float lam, multip;
     float c[MAXT];  // momentum coefficients
-    int nx, ny, margin, count;
-    bool nonneg, aniso, write_u, aligned;
+    bool nonneg, aniso, write_u;
 };
 
 // p scaled into the unit ball or clipped (utils.c:180-213)
@@ -49,10 +49,10 @@ __device__ __forceinline__ void project(float2& p1, float2& p2, bool aniso) {
 }
 
 template <int R, bool CHECK, bool DTV>
-__global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && !DTV && !CHECK) ? 2 : 1)
-    k_fgp_strip2d(Args a, const StopCtl* ctl, double2* partials) {
+__global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
+    k_fgp_strip2d(Args a, Frame fr) {
     __shared__ float2 first1[2][NW][32], first2[2][NW][32], last2[2][NW][32];
-    const Place<R> q(a.nx, a.ny, a.margin, a.aligned);
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w;
     // f and b never change during a run: loaded before the wait
     float2 f[R + 1], b1[DTV ? R : 1], b2[DTV ? R : 1];
@@ -65,17 +65,16 @@ __global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && 
             b2[r] = q.load_const(a.b[1], r);
         }
     }
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->stop) return;
-    float2 p1[R], p2[R], o1[R], o2[R], uo[CHECK ? R : 1];  // o: P^{k-2}, then R
+    if (!begin<CHECK>(fr)) return;
+    __shared__ float2 uo[CHECK ? R : 1][NW][32];  // U of the iteration before the check, each thread its own
+    float2 p1[R], p2[R], o1[R], o2[R];  // o: P^{k-2}, then R
 #pragma unroll
     for (int r = 0; r < R; r++) {
         p1[r] = a.pc[0] ? q.load(a.pc[0], r) : splat(0.f);
         p2[r] = a.pc[0] ? q.load(a.pc[1], r) : splat(0.f);
         o1[r] = a.pc[0] ? q.load(a.po[0], r) : splat(0.f);
         o2[r] = a.pc[0] ? q.load(a.po[1], r) : splat(0.f);
-        if (CHECK) uo[r] = a.count == 1 ? q.load(a.u, r) : splat(0.f);
+        if (CHECK && fr.count == 1) uo[CHECK ? r : 0][w][lane] = q.load(a.u_prev, r);
     }
     const float2 mlam2 = splat(-a.lam), mp2 = splat(a.multip);
     const bool top = q.Y == 0;
@@ -92,7 +91,7 @@ __global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && 
             if (a.nonneg) u = make_float2(u.x < 0.f ? 0.f : u.x, u.y < 0.f ? 0.f : u.y);
             return u;
         };
-        const bool last = t == a.count - 1;
+        const bool last = t == fr.count - 1;
         float2 u = u_of(o1[0], o2[0], r2up, f[0]);
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -116,10 +115,10 @@ __global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && 
             float2 n1 = fma2(mp2, g1, o1[r]), n2 = fma2(mp2, g2, o2[r]);
             project(n1, n2, a.aniso);
             if (last && a.write_u) {
-                if (CHECK) add_norms(q, r, u, uo[CHECK ? r : 0], pa, pb);
+                if (CHECK) add_norms(q, r, u, uo[CHECK ? r : 0][w][lane], pa, pb);
                 q.store(a.u, r, u);
             }
-            if (CHECK && t == a.count - 2) uo[CHECK ? r : 0] = u;
+            if (CHECK && t == fr.count - 2) uo[CHECK ? r : 0][w][lane] = u;
             o1[r] = p1[r];
             o2[r] = p2[r];
             p1[r] = n1;
@@ -127,7 +126,7 @@ __global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && 
             u = un;
         }
     };
-    for (int t = 0; t < a.count; t++) {
+    for (int t = 0; t < fr.count; t++) {
         const float2 cm = splat(a.c[t]);
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(NT, (R <= 2 && !(DTV && CHECK)) || (R == 3 && 
             q.store(a.qo[1], r, o2[r]);
         }
     }
-    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_fgp_strip2d<2, false, false>);
@@ -192,7 +191,7 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
     const bool checking = epsil != 0.0f;
     const Plan P = plan(d.nx, d.ny, iters, checking, b ? dtv : tv);
     Scratch scratch(s);
-    IterControl ctl(s, scratch, iters, epsil, P.nblocks);
+    IterControl ctl(s, scratch, iters, epsil, P.nblocks, 2);
     CILREG_TRY(ctl.status());
     const int nl = count_spans(iters, P.T, checking);
     // launch k writes (P, P before) to set[k & 1] and reads set[(k + 1) & 1]
@@ -205,24 +204,25 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
             }
     Args a = {};
     a.f = f;
-    a.u = u_out;
+    a.u_prev = u_out;
     a.lam = lam;
     a.multip = multip;
-    a.nx = d.nx;
-    a.ny = d.ny;
-    a.margin = P.margin;
     a.nonneg = nonneg;
     a.aniso = aniso;
-    a.aligned = host_aligned8(f) && host_aligned8(u_out);
+    bool aligned = host_aligned8(f) && host_aligned8(u_out);
     for (int c = 0; c < 2 && b; c++) {
         a.b[c] = b[c];
-        a.aligned = a.aligned && host_aligned8(b[c]);
+        aligned = aligned && host_aligned8(b[c]);
     }
     // a warm run starts from the newest duals of the caller's ring and leaves
     // its own in the buffer after it; its first coefficient is 0, so the
     // duals before the newest never count
     const int from = warm ? (warm->base + 2) % 3 : 0, to = warm ? warm->base : 0;
-    CILREG_TRY(for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
+    // U of a check must outlive the launch that carries the check: two buffers,
+    // of which the last launch writes u_out
+    float* ualt = checking && nl > 1 ? scratch.floats(d.n) : nullptr;
+    if (checking && nl > 1 && !ualt) return scratch.status();
+    CILREG_TRY(run_spans(P, ctl, iters, checking, d, aligned, [&](int k, const Span& sp, const Frame& fr) -> int {
         const bool end = k == nl - 1;
         for (int c = 0; c < 2; c++) {
             a.pc[c] = k > 0 ? set[(k + 1) & 1][c] : warm ? warm->ring[from][c] : nullptr;
@@ -235,17 +235,16 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
             }
         }
         for (int t = 0; t < sp.count; t++) a.c[t] = cseq[sp.first + t];
-        a.count = sp.count;
+        a.u = (checking && ((nl - 1 - k) & 1)) ? ualt : u_out;
         a.write_u = end || sp.check;
-        CILREG_CUDA(launch_pdl(b ? pick<true>(P.R, sp.check) : pick<false>(P.R, sp.check), P.grid, dim3(32, NW, 1), 0,
-                               s, a, (const StopCtl*)ctl.ctl(), ctl.partials()));
-        note_launch();
-        if (!sp.check) return 0;
-        CILREG_TRY(ctl.after_check(sp.first + sp.count - 1, P.nblocks));
-        return ctl.host_should_stop() ? 1 : 0;
+        CILREG_CUDA(launch_pdl(b ? pick<true>(P.R, checking) : pick<false>(P.R, checking), grid_of(P, fr, checking),
+                               dim3(32, NW, 1), 0, s, a, fr));
+        return OK;
     }));
     StopCtl done;
     CILREG_TRY(ctl.finish(info, &done));
+    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
+        CILREG_CUDA(cudaMemcpyAsync(u_out, ualt, sizeof(float) * (size_t)d.n, cudaMemcpyDeviceToDevice, s));
     if (warm && iters > 0) {
         if (checking) {
             const int k = done.stop ? span_of_check(done.iters) : nl - 1;

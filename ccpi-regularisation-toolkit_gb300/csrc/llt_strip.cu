@@ -17,19 +17,16 @@ using namespace strip;
 template <int R, bool CHECK>
 __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     k_llt_strip2d(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam_rof,
-                  float lam_llt, float tau, int nx, int ny, int margin, int count, bool aligned, const StopCtl* ctl,
-                  double2* partials) {
+                  float lam_llt, float tau, Frame fr) {
     __shared__ float2 first[2][2][NW][32], last[2][2][NW][32];  // [slot][row from the end]
-    const Place<R> q(nx, ny, margin, aligned);
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w;
     const float2 EPS2 = splat(1.0e-12f), MTWO2 = splat(-2.0f);
     const float2 tau2 = splat(tau), lrof2 = splat(lam_rof), mlllt2 = splat(-lam_llt);
     float2 f[R], u[R];
 #pragma unroll
     for (int r = 0; r < R; r++) f[r] = q.load_const(F, r);  // never changes: loaded before the wait
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->stop) return;
+    if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     float2 pa = splat(0.f), pb = splat(0.f);
@@ -108,7 +105,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
             um = c;
         }
     };
-    for (int t = 0; t < count; t++) {
+    for (int t = 0; t < fr.count; t++) {
         const int b = t & 1;
         first[b][0][w][lane] = u[0];
         first[b][1][w][lane] = u[1];
@@ -120,15 +117,15 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
         float2 below2 = lowest ? u[R - 1] : first[b][1][w + 1][lane];
         const float2 above = top ? u[1] : (w > 0 ? last[b][0][w - 1][lane] : u[0]);
         const float2 above_l = top ? u[0] : (w > 0 ? last[b][1][w - 1][lane] : u[0]);
-        const float2 above_h = top ? (ny == 2 ? u[0] : (R > 2 ? u[R > 2 ? 2 : 0] : below)) : u[0];
+        const float2 above_h = top ? (q.ny == 2 ? u[0] : (R > 2 ? u[R > 2 ? 2 : 0] : below)) : u[0];
         if (q.edge)
-            iterate(std::true_type{}, above_l, above, above_h, below, below2, t == count - 1);
+            iterate(std::true_type{}, above_l, above, above_h, below, below2, t == fr.count - 1);
         else
-            iterate(std::false_type{}, above_l, above, above_h, below, below2, t == count - 1);
+            iterate(std::false_type{}, above_l, above, above_h, below, below2, t == fr.count - 1);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_llt_strip2d<2, false>);
@@ -149,10 +146,9 @@ int llt_strip_run(const float* f, float* u_out, float lam_rof, float lam_llt, in
                   const Dims& d, cudaStream_t s, float* info) {
     static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 1600.0, 850.0};
     return run_flow(choices, f, f, u_out, iters, epsil, d, s, info, true,
-                    [&](const Plan& P, const Span& sp, const float* src, float* dst, bool aligned, IterControl& ctl) {
-                        return launch_pdl(pick(P, sp.check), P.grid, dim3(32, NW, 1), 0, s, src, dst, f, lam_rof,
-                                          lam_llt, tau, d.nx, d.ny, P.margin, sp.count, aligned,
-                                          (const StopCtl*)ctl.ctl(), ctl.partials());
+                    [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
+                        return launch_pdl(pick(P, rule), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam_rof,
+                                          lam_llt, tau, fr);
                     });
 }
 

@@ -15,17 +15,14 @@ using namespace strip;
 template <int PEN, int R, bool CHECK>
 __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
     k_ndf_strip2d(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam, float sg,
-                  float isg, float tau, int nx, int ny, int margin, int count, bool aligned, const StopCtl* ctl,
-                  double2* partials) {
+                  float isg, float tau, Frame fr) {
     __shared__ float2 first[2][NW][32], last[2][NW][32];
-    const Place<R> q(nx, ny, margin, aligned);
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w;
     float2 f[R], u[R];
 #pragma unroll
     for (int r = 0; r < R; r++) f[r] = q.load_const(F, r);  // never changes: loaded before the wait
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->stop) return;
+    if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     const float2 isg2 = splat(isg), lam2 = splat(lam), tau2 = splat(tau);
@@ -53,7 +50,7 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
             south = fy;
         }
     };
-    for (int t = 0; t < count; t++) {
+    for (int t = 0; t < fr.count; t++) {
         const int b = t & 1;
         first[b][w][lane] = u[0];
         last[b][w][lane] = u[R - 1];
@@ -61,13 +58,13 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         const float2 below = w < NW - 1 ? first[b][w + 1][lane] : u[R - 1];
         const float2 above = q.Y == 0 ? u[1] : (w > 0 ? last[b][w - 1][lane] : u[0]);
         if (q.edge)
-            iterate(std::true_type{}, above, below, t == count - 1);
+            iterate(std::true_type{}, above, below, t == fr.count - 1);
         else
-            iterate(std::false_type{}, above, below, t == count - 1);
+            iterate(std::false_type{}, above, below, t == fr.count - 1);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_ndf_strip2d<0, 2, false>);
@@ -99,10 +96,9 @@ int ndf_strip_run(int pen, const float* f, float* u_out, float lam, float sg, fl
                   float epsil, const Dims& d, cudaStream_t s, float* info, const float* u_init) {
     static const Choices choices = {1, 3, {2, 4, 6}, {2, 2, 1}, 500.0, 250.0};
     return run_flow(choices, f, u_init ? u_init : f, u_out, iters, epsil, d, s, info, true,
-                    [&](const Plan& P, const Span& sp, const float* src, float* dst, bool aligned, IterControl& ctl) {
-                        return launch_pdl(pick(pen, P, sp.check), P.grid, dim3(32, NW, 1), 0, s, src, dst, f, lam, sg,
-                                          isg, tau, d.nx, d.ny, P.margin, sp.count, aligned,
-                                          (const StopCtl*)ctl.ctl(), ctl.partials());
+                    [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
+                        return launch_pdl(pick(pen, P, rule), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam, sg,
+                                          isg, tau, fr);
                     });
 }
 

@@ -30,10 +30,9 @@ __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
 template <int R, bool CHECK, bool LARR>
 __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
     k_rof_strip2d(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F,
-                  const float* __restrict__ lam_arr, float lam, float tau, int nx, int ny, int margin, int count,
-                  bool aligned, const StopCtl* ctl, double2* partials) {
+                  const float* __restrict__ lam_arr, float lam, float tau, Frame fr) {
     __shared__ float2 first[2][NW][32], last[2][NW][32];
-    const Place<R> q(nx, ny, margin, aligned);
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w, Y = q.Y;
     // f and the lambda map never change during a run: loaded before waiting
     // for the previous launch (launch_pdl)
@@ -44,9 +43,7 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         if (LARR) l[r] = q.load_const(lam_arr, r);
     }
     if (!LARR) l[0] = splat(lam);
-    pdl_wait();
-    pdl_trigger();
-    if (ctl->stop) return;
+    if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     const float2 EPS2 = splat(1.0e-8f), tau2 = splat(tau);
@@ -94,7 +91,7 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
             d1l = d1;
         }
     };
-    for (int t = 0; t < count; t++) {
+    for (int t = 0; t < fr.count; t++) {
         const int b = t & 1;
         first[b][w][lane] = u[0];
         last[b][w][lane] = u[R - 1];
@@ -103,13 +100,13 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         const float2 above = Y == 0 ? u[1] : (w > 0 ? last[b][w - 1][lane] : u[0]);
         const float2 next = Y == 0 ? (R > 2 ? u[R > 2 ? 2 : 0] : below) : u[0];
         if (q.edge)
-            iterate(std::true_type{}, above, ny == 2 && Y == 0 ? u[0] : next, below, t == count - 1);
+            iterate(std::true_type{}, above, q.ny == 2 && Y == 0 ? u[0] : next, below, t == fr.count - 1);
         else
-            iterate(std::false_type{}, above, next, below, t == count - 1);
+            iterate(std::false_type{}, above, next, below, t == fr.count - 1);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) block_pair_partial<NT>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_rof_strip2d<2, false, false>);
@@ -135,10 +132,9 @@ int rof_strip_run(const float* f, float* u_out, const float* lam_arr, float lam,
     static const Choices choices = {1, 4, {2, 3, 4, 6}, {2, 2, 2, 1}, 660.0, 300.0};
     const bool larr = lam_arr != nullptr;
     return run_flow(choices, f, u_init ? u_init : f, u_out, iters, epsil, d, s, info, !larr || host_aligned8(lam_arr),
-                    [&](const Plan& P, const Span& sp, const float* src, float* dst, bool aligned, IterControl& ctl) {
-                        return launch_pdl(pick(P, sp.check, larr), P.grid, dim3(32, NW, 1), 0, s, src, dst, f, lam_arr,
-                                          lam, tau, d.nx, d.ny, P.margin, sp.count, aligned,
-                                          (const StopCtl*)ctl.ctl(), ctl.partials());
+                    [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
+                        return launch_pdl(pick(P, rule, larr), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam_arr,
+                                          lam, tau, fr);
                     });
 }
 

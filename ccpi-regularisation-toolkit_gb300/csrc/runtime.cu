@@ -204,51 +204,10 @@ __global__ void k_init_ctl(StopCtl* c, int iters) {
 // the stopping control of runs without a rule: never set, never written
 __device__ StopCtl g_running;
 
-// Deterministic reduction of the per-CTA FP64 partials, then the stopping
-// rule.  One CTA of 1024 threads; fixed assignment of partials to threads.
-// `mirror` (may be null): the host's copy, written here instead of by a copy
-// and an event per check, which kept the next iteration from starting for
-// about 15 us (512^2 images with a check every 5 iterations: 23 us per check
-// before, 9-11 now).
-__global__ void __launch_bounds__(1024) k_finalize_check(const double2* __restrict__ part, long long nparts,
-                                                          StopCtl* ctl, float epsil, int it, StopMirror* mirror,
-                                                          int seq) {
+__global__ void __launch_bounds__(1024) k_finalize_check(Finalize f) {
     pdl_wait();  // the check iteration has completed (launch_pdl)
     pdl_trigger();
-    if (ctl->stop) return;
-    double a = 0.0, b = 0.0;
-    for (long long p = threadIdx.x; p < nparts; p += 1024) {
-        double2 v = part[p];
-        a += v.x;
-        b += v.y;
-    }
-    __shared__ double sa[32], sb[32];
-    a = warp_sum(a);
-    b = warp_sum(b);
-    if ((threadIdx.x & 31) == 0) { sa[threadIdx.x >> 5] = a; sb[threadIdx.x >> 5] = b; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        a = warp_sum(sa[threadIdx.x]);
-        b = warp_sum(sb[threadIdx.x]);
-        if (threadIdx.x == 0) {
-            float re = sqrtf((float)a) / sqrtf((float)b);
-            StopCtl c = *ctl;
-            c.re = re;
-            if (re < epsil) c.count += 1;
-            if (c.count > 3) {
-                c.stop = 1;
-                c.iters = it;
-            }
-            *ctl = c;
-            if (mirror) {
-                *(volatile int*)&mirror->ctl.stop = c.stop;
-                *(volatile int*)&mirror->ctl.iters = c.iters;
-                *(volatile int*)&mirror->ctl.count = c.count;
-                *(volatile float*)&mirror->ctl.re = c.re;
-                asm volatile("st.release.sys.global.b32 [%0], %1;" ::"l"(&mirror->seq), "r"(seq) : "memory");
-            }
-        }
-    }
+    finalize_check<1024>(f);
 }
 
 namespace {
@@ -300,8 +259,9 @@ StopCtl* running_ctl() {
 
 }  // namespace
 
-IterControl::IterControl(cudaStream_t s, Scratch& scratch, int iter_total, float epsil, long long max_partials)
-    : stream_(s), iter_total_(iter_total), epsil_(epsil) {
+IterControl::IterControl(cudaStream_t s, Scratch& scratch, int iter_total, float epsil, long long max_partials,
+                         int partial_sets)
+    : stream_(s), slots_(max_partials < 1 ? 1 : max_partials), iter_total_(iter_total), epsil_(epsil) {
     if (epsil == 0.0f) {  // no rule: nothing to allocate, initialise or read back
         d_ctl_ = running_ctl();
         if (!d_ctl_) status_ = fail(ERR_CUDA, __FILE__, __LINE__, "no address for the stop control");
@@ -309,7 +269,7 @@ IterControl::IterControl(cudaStream_t s, Scratch& scratch, int iter_total, float
     }
     d_ctl_ = (StopCtl*)scratch.bytes(sizeof(StopCtl));
     if (!d_ctl_) { status_ = scratch.status(); return; }
-    d_part_ = (double2*)scratch.bytes(sizeof(double2) * (size_t)(max_partials < 1 ? 1 : max_partials));
+    d_part_ = (double2*)scratch.bytes(sizeof(double2) * (size_t)slots_ * partial_sets);
     if (!d_part_) { status_ = scratch.status(); return; }
     k_init_ctl<<<1, 1, 0, s>>>(d_ctl_, iter_total);
     note_launch();
@@ -332,11 +292,14 @@ IterControl::~IterControl() {
     }
 }
 
-int IterControl::after_check(int it, long long nparts) {
-    CILREG_CUDA(launch_pdl(k_finalize_check, dim3(1), dim3(1024), 0, stream_, (const double2*)d_part_, nparts, d_ctl_,
-                           epsil_, it, h_, checks_ + 1));
-    note_launch();
+Finalize IterControl::fold_check(int it, long long nparts, int k) {
     checks_++;
+    return Finalize{partials(k), nparts, d_ctl_, epsil_, it, h_, checks_};
+}
+
+int IterControl::after_check(int it, long long nparts, int k) {
+    CILREG_CUDA(launch_pdl(k_finalize_check, dim3(1), dim3(1024), 0, stream_, fold_check(it, nparts, k)));
+    note_launch();
     return OK;
 }
 
@@ -463,7 +426,7 @@ int launch_init_ctl(StopCtl* ctl, int iter_total, cudaStream_t s) {
 
 int launch_finalize_check(const double2* partials, long long nparts, StopCtl* ctl, float epsil, int it,
                           cudaStream_t s) {
-    k_finalize_check<<<1, 1024, 0, s>>>(partials, nparts, ctl, epsil, it, nullptr, 0);
+    k_finalize_check<<<1, 1024, 0, s>>>(Finalize{partials, nparts, ctl, epsil, it, nullptr, 0});
     CILREG_CUDA(cudaGetLastError());
     note_launch();
     return OK;

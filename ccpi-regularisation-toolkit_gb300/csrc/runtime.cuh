@@ -104,10 +104,23 @@ struct StopMirror {
     int seq;
 };
 
+// One check to reduce: its partials (n = 0: none) and where the rule's outcome goes.
+struct Finalize {
+    const double2* part;
+    long long n;
+    StopCtl* ctl;
+    float epsil;
+    int it;              // the check's iteration
+    StopMirror* mirror;  // may be null
+    int seq;             // the check's number
+};
+
 // Device-resident stopping control for one regulariser run.
 class IterControl {
 public:
-    IterControl(cudaStream_t s, Scratch& scratch, int iter_total, float epsil, long long max_partials);
+    // partial_sets: 2 for runs that fold their checks
+    IterControl(cudaStream_t s, Scratch& scratch, int iter_total, float epsil, long long max_partials,
+                int partial_sets = 1);
     ~IterControl();
     int status() const { return status_; }
     StopCtl* ctl() const { return d_ctl_; }
@@ -116,7 +129,12 @@ public:
     // the reference's test: a check happens at iteration `it` when it % 5 == 0
     bool is_check(int it) const { return epsil_ != 0.0f && (it % 5) == 0; }
     // enqueue the reduction of `nparts` partials for iteration `it`
-    int after_check(int it, long long nparts);
+    int after_check(int it, long long nparts, int k = 0);
+    // the same check as an argument for the next launch, one CTA of which
+    // runs it (finalize_check) beside that launch's own work; launch k's
+    // partials then lie in slot k & 1
+    Finalize fold_check(int it, long long nparts, int k);
+    double2* partials(int k) const { return d_part_ ? d_part_ + (k & 1) * slots_ : nullptr; }
     // true when the host may stop enqueueing (the rule has fired on device)
     bool host_should_stop();
     // wait for completion and fill infovector[0..1] (host pointer, may be null)
@@ -128,6 +146,7 @@ private:
     double2* d_part_ = nullptr;
     StopMirror* h_ = nullptr;  // page-locked, written by the device
     int checks_ = 0;           // checks enqueued
+    long long slots_ = 0;
     int iter_total_;
     float epsil_;
     int status_ = 0;
@@ -185,6 +204,49 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ((KArgs)args)...);
     cudaGetLastError();  // the status is returned; leave no stale error behind
     return e;
+}
+
+// Deterministic reduction of a check's FP64 partials by one CTA of THREADS
+// threads (a fixed assignment of partials to threads), then the stopping rule
+// and the host's copy of it, written here instead of by a copy and an event
+// per check, which kept the next iteration from starting for about 10 us.
+template <int THREADS>
+__device__ __forceinline__ void finalize_check(const Finalize& f) {
+    if (f.ctl->stop) return;
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    double a = 0.0, b = 0.0;
+    for (long long p = tid; p < f.n; p += THREADS) {
+        const double2 v = f.part[p];
+        a += v.x;
+        b += v.y;
+    }
+    __shared__ double sa[32], sb[32];
+    a = warp_sum(a);
+    b = warp_sum(b);
+    if ((tid & 31) == 0) { sa[tid >> 5] = a; sb[tid >> 5] = b; }
+    __syncthreads();
+    if (tid < 32) {
+        a = warp_sum(tid < THREADS / 32 ? sa[tid] : 0.0);
+        b = warp_sum(tid < THREADS / 32 ? sb[tid] : 0.0);
+        if (tid == 0) {
+            const float re = sqrtf((float)a) / sqrtf((float)b);
+            StopCtl c = *f.ctl;
+            c.re = re;
+            if (re < f.epsil) c.count += 1;
+            if (c.count > 3) {
+                c.stop = 1;
+                c.iters = f.it;
+            }
+            *f.ctl = c;
+            if (f.mirror) {
+                *(volatile int*)&f.mirror->ctl.stop = c.stop;
+                *(volatile int*)&f.mirror->ctl.iters = c.iters;
+                *(volatile int*)&f.mirror->ctl.count = c.count;
+                *(volatile float*)&f.mirror->ctl.re = c.re;
+                asm volatile("st.release.sys.global.b32 [%0], %1;" ::"l"(&f.mirror->seq), "r"(f.seq) : "memory");
+            }
+        }
+    }
 }
 
 // process-wide count of kernels this library has launched (for benchmarks)

@@ -40,7 +40,7 @@ struct Plan {
     int R = 0;       // rows per thread; 0: the image does not run strips
     int T = 0;       // most iterations per launch
     int margin = 0;  // halo of the tiles
-    dim3 grid;
+    int gx = 0, gy = 0;  // tiles along x and y
     long long nblocks = 0;
 };
 
@@ -106,7 +106,8 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
                     best.R = R;
                     best.T = t;
                     best.margin = m;
-                    best.grid = dim3((unsigned)tiles(nx, SW, m), (unsigned)tiles(ny, H, m), 1);
+                    best.gx = tiles(nx, SW, m);
+                    best.gy = tiles(ny, H, m);
                     best.nblocks = nb;
                 }
             }
@@ -114,6 +115,59 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
         if (best.R) return best;
     }
     return Plan{};
+}
+
+// What every launch gets besides its arrays: the image, the tiles, and the
+// check of the launch before, which CTA 0 then reduces while the others run.
+// The stop it may set holds from the launch after this one on, whose tiles
+// then leave both launches' results alone: launch k and k+1 write different
+// buffers, so a run that stops at launch k's check ends on k's.  (A finalize
+// kernel between them cost 7 us per check.)  RULE: the run has a stopping rule;
+// the kernels of runs without one are compiled without all of this, which
+// would cost them 3 to 10%.
+struct Frame {
+    int nx, ny, margin, count, gx;
+    bool aligned;
+    const StopCtl* ctl;
+    double2* partials;
+    Finalize check;
+};
+template <bool RULE>
+__device__ __forceinline__ int tile_index(const Frame& F) {
+    return (int)blockIdx.x - (RULE && F.check.n > 0 ? 1 : 0);
+}
+// waits for the launch before; false where the CTA has no tile to run
+template <bool RULE>
+__device__ __forceinline__ bool begin(const Frame& F) {
+    pdl_wait();
+    pdl_trigger();
+    if (!RULE) return true;
+    if (tile_index<RULE>(F) < 0) {
+        finalize_check<NT>(F.check);
+        return false;
+    }
+    return !F.ctl->stop;
+}
+inline dim3 grid_of(const Plan& P, const Frame& F, bool rule) {
+    return rule ? dim3((unsigned)(P.nblocks + (F.check.n > 0 ? 1 : 0))) : dim3((unsigned)P.gx, (unsigned)P.gy);
+}
+// one FP64 partial of the CTA's FP32 sums.  Two warps add the threads' sums
+// from shared memory: the FP64 unit takes 16 cycles for a warp's addition, and
+// a shuffle reduction of both sums in every warp is 170 of them per CTA
+// against 42.
+__device__ __forceinline__ void store_partial(float a, float b, double2* slot) {
+    __shared__ float sum[2][NT];
+    const int lane = threadIdx.x, w = threadIdx.y;
+    sum[0][w * 32 + lane] = a;
+    sum[1][w * 32 + lane] = b;
+    __syncthreads();
+    if (w < 2) {
+        double v = 0.0;
+#pragma unroll
+        for (int j = 0; j < NW; j++) v += (double)sum[w][j * 32 + lane];
+        v = warp_sum(v);
+        if (lane == 0) (w == 0 ? slot->x : slot->y) = v;
+    }
 }
 
 // a thread's place in its tile and what it may store
@@ -129,11 +183,13 @@ struct Place {
     int bottom;      // the strip's row that is the image's last, if any
     int c0, c1;      // columns clamped into the image
     bool vec;        // 8-byte accesses
-    __device__ __forceinline__ Place(int nx_, int ny_, int margin, bool aligned) : nx(nx_), ny(ny_) {
+    __device__ __forceinline__ Place(const Frame& F, bool rule, int tile) : nx(F.nx), ny(F.ny) {
         constexpr int H = NW * R;
+        const int margin = F.margin;
         lane = threadIdx.x;
         w = threadIdx.y;
-        const int X0 = blockIdx.x * (SW - 2 * margin), Y0 = blockIdx.y * (H - 2 * margin);
+        const int bx = rule ? tile % F.gx : blockIdx.x, by = rule ? tile / F.gx : blockIdx.y;
+        const int X0 = bx * (SW - 2 * margin), Y0 = by * (H - 2 * margin);
         X = X0 + 2 * lane;
         Y = Y0 + w * R;
         const int xa = X0 ? X0 + margin : 0, xb = (X0 + SW >= nx) ? nx : X0 + SW - margin;
@@ -146,7 +202,7 @@ struct Place {
         at_right = X + 2 == nx;
         odd_end = X + 1 == nx;
         bottom = ny - 1 - Y;
-        vec = aligned && (nx & 1) == 0;
+        vec = F.aligned && (nx & 1) == 0;
         c0 = vec ? min(X, nx - 2) : min(X, nx - 1);
         c1 = min(X + 1, nx - 1);
     }
@@ -250,17 +306,36 @@ __device__ __forceinline__ void add_norms(const Place<R>& q, int r, float2 un, f
     pb = fma2(um, um, pb);
 }
 
+// The launches of a run: each(k, span, frame) enqueues launch k.  The check of
+// launch k rides on launch k+1, the last launch's gets a kernel of its own.
+template <class F>
+int run_spans(const Plan& P, IterControl& ctl, int iters, bool checking, const Dims& d, bool aligned, F each) {
+    const int nl = count_spans(iters, P.T, checking);
+    Finalize pending = {};
+    return for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
+        const Frame fr{d.nx, d.ny, P.margin, sp.count, P.gx, aligned, ctl.ctl(), ctl.partials(k), pending};
+        CILREG_TRY(each(k, sp, fr));
+        note_launch();
+        pending = Finalize{};
+        if (!sp.check) return 0;
+        const int it = sp.first + sp.count - 1;
+        if (k == nl - 1) return ctl.after_check(it, P.nblocks, k);
+        pending = ctl.fold_check(it, P.nblocks, k);
+        return ctl.host_should_stop() ? 1 : 0;
+    });
+}
+
 // The run of a regulariser whose state is one image U beside f (ROF, NDF,
-// Diff4th, LLT-ROF): launch(plan, span, src, dst, aligned, ctl) enqueues one
-// launch.  Launch k writes bufs[(nl - 1 - k) & 1], so the last writes u_out;
-// a run that stops early on the other buffer copies it.
+// Diff4th, LLT-ROF): launch(plan, rule, frame, src, dst) enqueues one launch.
+// Launch k writes bufs[(nl - 1 - k) & 1], so the last writes u_out; a run that
+// stops early on the other buffer copies it.
 template <class Launch>
 int run_flow(const Choices& choices, const float* f, const float* start, float* u_out, int iters, float epsil,
              const Dims& d, cudaStream_t s, float* info, bool aligned, Launch launch) {
     const bool checking = epsil != 0.0f;
     const Plan P = plan(d.nx, d.ny, iters, checking, choices);
     Scratch scratch(s);
-    IterControl ctl(s, scratch, iters, epsil, P.nblocks);
+    IterControl ctl(s, scratch, iters, epsil, P.nblocks, 2);
     CILREG_TRY(ctl.status());
     const size_t bytes = sizeof(float) * (size_t)d.n;
     if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, start, bytes, cudaMemcpyDeviceToDevice, s));
@@ -269,13 +344,9 @@ int run_flow(const Choices& choices, const float* f, const float* start, float* 
     if (nl > 1 && !alt) return scratch.status();
     float* bufs[2] = {u_out, alt};
     aligned = aligned && host_aligned8(f) && host_aligned8(start) && host_aligned8(u_out);
-    CILREG_TRY(for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
-        const float* src = k == 0 ? start : bufs[(nl - k) & 1];
-        CILREG_CUDA(launch(P, sp, src, bufs[(nl - 1 - k) & 1], aligned, ctl));
-        note_launch();
-        if (!sp.check) return 0;
-        CILREG_TRY(ctl.after_check(sp.first + sp.count - 1, P.nblocks));
-        return ctl.host_should_stop() ? 1 : 0;
+    CILREG_TRY(run_spans(P, ctl, iters, checking, d, aligned, [&](int k, const Span&, const Frame& fr) -> int {
+        CILREG_CUDA(launch(P, checking, fr, k == 0 ? start : bufs[(nl - k) & 1], bufs[(nl - 1 - k) & 1]));
+        return OK;
     }));
     StopCtl done;
     CILREG_TRY(ctl.finish(info, &done));
