@@ -110,6 +110,13 @@ int pd_run(const float* f, float* u_out, float lam, int iters, float epsil, floa
     CILREG_RANGE("cilreg PD-TV");
     const bool three = d.nz > 1;
     const int nc = three ? 3 : 2;
+    // step sizes (PD_TV_core.c:50-53): sigma = 1/(L tau) formed in double
+    const float tau = lam * 0.1f;
+    const float sigma = (float)(1.0 / (double)(lipschitz * tau));
+    const float lt = tau / lam;
+    const DoubleDivisor onelt = make_double_divisor(1.0 + (double)lt);  // the reference divides by (1.0 + lt)
+    if (pd_strip_applies(d))
+        return pd_strip_run(f, u_out, sigma, tau, lt, onelt, iters, epsil, nonneg == 1, methodTV != 0, d, s, info);
     Scratch scratch(s);
     const Launch3 L = plan_launch(d);
     // CILREG_PD_KERNEL=simple selects the per-voxel kernel (kept for A/B checks)
@@ -133,11 +140,6 @@ int pd_run(const float* f, float* u_out, float lam, int iters, float epsil, floa
     for (int c = 0; c < nc; c++) CILREG_CUDA(cudaMemsetAsync(pb[0][c], 0, sizeof(float) * d.n, s));
     if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, f, sizeof(float) * d.n, cudaMemcpyDeviceToDevice, s));
 
-    // step sizes (PD_TV_core.c:50-53): sigma = 1/(L tau) formed in double
-    const float tau = lam * 0.1f;
-    const float sigma = (float)(1.0 / (double)(lipschitz * tau));
-    const float lt = tau / lam;
-    const DoubleDivisor onelt = make_double_divisor(1.0 + (double)lt);  // the reference divides by (1.0 + lt)
     int it = 0;
     if (stream && !ctl.checking() && d.n <= (1LL << 22)) {
         // small volume, fixed count: launch overhead dominates, replay a graph

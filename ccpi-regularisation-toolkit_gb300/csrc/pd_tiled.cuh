@@ -28,4 +28,10 @@ PdPlan pd_stream_plan(const Dims& d);
 int pd_stream_step(const PdPlan& T, const PdStreamArgs& a, const Dims& d, const StopCtl* ctl, double2* partials,
                    cudaStream_t s);
 
+// 2D images run several iterations per launch (pd_strip.cu; CILREG_PD_KERNEL or
+// CILREG_STRIP2D=0 keep one per launch)
+bool pd_strip_applies(const Dims& d);
+int pd_strip_run(const float* f, float* u_out, float sigma, float tau, float lt, const DoubleDivisor& onelt, int iters,
+                 float epsil, bool nonneg, bool aniso, const Dims& d, cudaStream_t s, float* info);
+
 }  // namespace cilreg
