@@ -137,8 +137,39 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
     CILREG_RANGE("cilreg SB-TV");
     const bool three = d.nz > 1;
     const int nc = three ? 3 : 2;
-    Scratch scratch(s);
     const Launch3 L = plan_launch(d);
+    if (sb_strip_applies(d)) {
+        SbSweepArgs in = {};
+        in.f = f;
+        in.mu = 1.0f / mu;  // mu <- 1/mu, lambda = 2 mu (SB_TV_core.c:45-46)
+        in.lambda = 2.0f * in.mu;
+        in.norm = 1.0f / (in.mu + 4.0f * in.lambda);
+        const float dlam = 1.0f / in.lambda;
+        CILREG_TRY(sb_strip_run(in, dlam, methodTV == 1, u_out, iters, epsil, d, s, info, warm));
+        if (warm && iters > 0) {  // D^n, B^n from the final U, in place
+            Scratch tmp(s);
+            StopCtl* never = (StopCtl*)tmp.bytes(sizeof(StopCtl));
+            if (!never) return tmp.status();
+            CILREG_CUDA(cudaMemsetAsync(never, 0, sizeof(StopCtl), s));
+            SbArgs a = {};
+            for (int c = 0; c < 2; c++) {
+                a.dd[c] = warm->dd[c];
+                a.bb[c] = warm->bb[c];
+            }
+            a.u = u_out;
+            a.lambda = in.lambda;
+            a.mu = in.mu;
+            a.norm = in.norm;
+            a.dlam = dlam;
+            a.aniso = (methodTV == 1);
+            a.f = f;
+            k_sb_shrink<false><<<L.grid, L.block, 0, s>>>(a, d, L.kz, never);
+            CILREG_CUDA(cudaGetLastError());
+            note_launch();
+        }
+        return OK;
+    }
+    Scratch scratch(s);
     const SbPlan T = sb_sweep2_plan(d);
     const long long nparts = T.use ? T.nblocks : num_blocks(L);
     IterControl ctl(s, scratch, iters, epsil, nparts);

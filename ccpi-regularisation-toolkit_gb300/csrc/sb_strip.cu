@@ -1,0 +1,239 @@
+// Split-Bregman TV on 2D images, several outer iterations per launch
+// (strip2d.cuh).  As in k_sb_fused, the state is (U^k, B^{k-1}): an iteration
+// forms D^k, B^k from it and runs both Jacobi sweeps (SB_TV_core.c:149-371).
+// The shrinkage of the row above a strip is recomputed from that row's U and
+// B; the first sweep's U1 is exchanged after a second barrier.
+#include "sb_tiled.cuh"
+#include "strip2d.cuh"
+
+namespace cilreg {
+
+namespace {
+
+using namespace strip;
+
+struct Args {
+    const float* u;      // U^k
+    float* un;           // U after the launch
+    const float* bp[2];  // B^{k-1}; of the first iteration: B^0, null for zero
+    const float* d0[2];  // of the first iteration: D^0, null for zero
+    float* bn[2];        // B after the launch; null: not stored
+    const float* f;
+    float lambda, mu, norm, dlam;
+    bool first;  // the launch starts with iteration 0, whose D and B are given
+    bool aniso;
+};
+
+// D = shrink(g + b) and B = b + (g - D) of a pair
+__device__ __forceinline__ void shrink(float2 g1, float2 g2, float2 b1, float2 b2, float dlam, bool aniso, float2& d1,
+                                       float2& d2, float2& n1, float2& n2) {
+    const float2 v1 = add2(g1, b1), v2 = add2(g2, b2);
+    if (aniso) {
+        // (v / |v|) * max(|v| - 1/lambda, 0), 0 for v == 0: the same value as a sign copy
+        auto one = [&](float v) { return copysignf(fmaxf(fabsf(v) - dlam, 0.f), v); };
+        d1 = make_float2(one(v1.x), one(v1.y));
+        d2 = make_float2(one(v2.x), one(v2.y));
+    } else {
+        const float2 sq = fma2(v1, v1, mul2(v2, v2));
+        const float2 den = make_float2(__fsqrt_rn(sq.x), __fsqrt_rn(sq.y));
+        const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
+        const float2 r = make_float2(den.x != 0.f ? __frcp_rn(den.x) : 0.f, den.y != 0.f ? __frcp_rn(den.y) : 0.f);
+        d1 = mul2(m, mul2(v1, r));
+        d2 = mul2(m, mul2(v2, r));
+    }
+    n1 = add2(b1, sub2(g1, d1));
+    n2 = add2(b2, sub2(g2, d2));
+}
+
+template <int R, bool CHECK>
+__global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame fr) {
+    __shared__ float2 firstU[NW][32], lastU[NW][32], lastB1[NW][32], lastB2[NW][32], first1[NW][32], last1[NW][32];
+    const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
+    const int lane = q.lane, w = q.w;
+    float2 muf[R], u[R], b1[R], b2[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) muf[r] = mul2(splat(a.mu), q.load_const(a.f, r));  // before the wait
+    if (!begin<CHECK>(fr)) return;
+    const bool top = q.Y == 0;
+    float2 d1[R], d2[R], d2up = splat(0.f), b2up = splat(0.f);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        u[r] = q.load(a.u, r);
+        b1[r] = a.bp[0] ? q.load(a.bp[0], r) : splat(0.f);
+        b2[r] = a.bp[0] ? q.load(a.bp[1], r) : splat(0.f);
+        d1[r] = d2[r] = splat(0.f);
+    }
+    if (a.first && a.d0[0]) {  // given D^0, B^0: of the rows and of the one above
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            d1[r] = q.load(a.d0[0], r);
+            d2[r] = q.load(a.d0[1], r);
+        }
+        const int up = top ? 1 : -1;  // row -1 of the image is the mirrored row 1
+        d2up = q.load(a.d0[1], up);
+        b2up = q.load(a.bp[1], up);
+    }
+    const float2 lam2 = splat(a.lambda), norm2 = splat(a.norm);
+    float2 pa = splat(0.f), pb = splat(0.f);
+    float2 g[R], u1[R];
+
+    auto sum4 = [](float2 xh, float2 xl, float2 yh, float2 yl) { return add2(add2(add2(xh, xl), yh), yl); };
+    // D, B, their divergence term G and the first sweep
+    auto sweep1 = [&](auto edge_, float2 above, float2 next, float2 below, float2 b1a, float2 b2a, bool given) {
+        constexpr bool EDGE = decltype(edge_)::value;
+        if (!given) {  // the row above: D2 and B2
+            float2 c = above, e1, n1;
+            float lo, hi;
+            x_neighbours<EDGE>(q, c, lo, hi);
+            shrink(sub2(make_float2(c.y, hi), c), sub2(next, c), b1a, b2a, a.dlam, a.aniso, e1, d2up, n1, b2up);
+        }
+        float2 um = above, dl = d2up, bl = b2up;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            float2 c = u[r];
+            float lo, hi;
+            x_neighbours<EDGE>(q, c, lo, hi);
+            const float2 xl = make_float2(lo, c.x), xh = make_float2(c.y, hi);
+            float2 uh = (r < R - 1) ? u[r + 1 < R ? r + 1 : r] : below;
+            if (EDGE && r == q.bottom) uh = um;
+            if (!given) {
+                float2 n1, n2;
+                shrink(sub2(xh, c), sub2(uh, c), b1[r], b2[r], a.dlam, a.aniso, d1[r], d2[r], n1, n2);
+                b1[r] = n1;
+                b2[r] = n2;
+            }
+            float dxl = left_of(d1[r]), bxl = left_of(b1[r]);
+            if (EDGE && q.at_left) {
+                dxl = d1[r].y;
+                bxl = b1[r].y;
+            }
+            // Dx[-1] - Dx + Dy[-1] - Dy - Bx[-1] + Bx - By[-1] + By (SB_TV_core.c:166)
+            float2 s = sub2(make_float2(dxl, d1[r].x), d1[r]);
+            s = sub2(add2(s, dl), d2[r]);
+            s = add2(sub2(s, make_float2(bxl, b1[r].x)), b1[r]);
+            s = add2(sub2(s, bl), b2[r]);
+            g[r] = s;
+            u1[r] = mul2(norm2, fma2(add2(s, sum4(xh, xl, uh, um)), lam2, muf[r]));
+            um = u[r];
+            dl = d2[r];
+            bl = b2[r];
+        }
+    };
+    auto sweep2 = [&](auto edge_, float2 above, float2 below, bool sum) {
+        constexpr bool EDGE = decltype(edge_)::value;
+        float2 um = above;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            float2 c = u1[r];
+            float lo, hi;
+            x_neighbours<EDGE>(q, c, lo, hi);
+            float2 uh = (r < R - 1) ? u1[r + 1 < R ? r + 1 : r] : below;
+            if (EDGE && r == q.bottom) uh = um;
+            const float2 s = add2(g[r], sum4(make_float2(c.y, hi), make_float2(lo, c.x), uh, um));
+            const float2 un = mul2(norm2, fma2(s, lam2, muf[r]));
+            if (CHECK && sum) add_norms(q, r, un, u1[r], pa, pb);
+            u[r] = un;
+            um = u1[r];
+        }
+    };
+    for (int t = 0; t < fr.count; t++) {
+        firstU[w][lane] = u[0];
+        lastU[w][lane] = u[R - 1];
+        lastB1[w][lane] = b1[R - 1];
+        lastB2[w][lane] = b2[R - 1];
+        __syncthreads();
+        const float2 below = w < NW - 1 ? firstU[w + 1][lane] : u[R - 1];
+        const float2 above = top ? u[1] : (w > 0 ? lastU[w - 1][lane] : u[0]);
+        const float2 next = top ? (q.ny == 2 ? u[0] : (R > 2 ? u[R > 2 ? 2 : 0] : below)) : u[0];
+        const float2 b1a = top ? b1[1] : (w > 0 ? lastB1[w - 1][lane] : b1[0]);
+        const float2 b2a = top ? b2[1] : (w > 0 ? lastB2[w - 1][lane] : b2[0]);
+        const bool given = a.first && t == 0;
+        if (q.edge)
+            sweep1(std::true_type{}, above, next, below, b1a, b2a, given);
+        else
+            sweep1(std::false_type{}, above, next, below, b1a, b2a, given);
+        first1[w][lane] = u1[0];
+        last1[w][lane] = u1[R - 1];
+        __syncthreads();
+        const float2 below1 = w < NW - 1 ? first1[w + 1][lane] : u1[R - 1];
+        const float2 above1 = top ? u1[1] : (w > 0 ? last1[w - 1][lane] : u1[0]);
+        if (q.edge)
+            sweep2(std::true_type{}, above1, below1, t == fr.count - 1);
+        else
+            sweep2(std::false_type{}, above1, below1, t == fr.count - 1);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        q.store(a.un, r, u[r]);
+        if (a.bn[0]) {
+            q.store(a.bn[0], r, b1[r]);
+            q.store(a.bn[1], r, b2[r]);
+        }
+    }
+    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+}
+
+using Kernel = decltype(&k_sb_strip2d<2, false>);
+Kernel pick(int R, bool rule) {
+    if (R == 2) return rule ? k_sb_strip2d<2, true> : k_sb_strip2d<2, false>;
+    if (R == 3) return rule ? k_sb_strip2d<3, true> : k_sb_strip2d<3, false>;
+    return rule ? k_sb_strip2d<4, true> : k_sb_strip2d<4, false>;
+}
+
+}  // namespace
+
+bool sb_strip_applies(const Dims& d) {
+    const char* ek = getenv("CILREG_SB_KERNEL");
+    return strip::applies(d) && !(ek && ek[0] != '\0');
+}
+
+int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, int iters, float epsil, const Dims& d,
+                 cudaStream_t s, float* info, SbWarm* warm) {
+    static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 1620.0, 685.0, 1000.0, 800.0};
+    const bool checking = epsil != 0.0f;
+    const Plan P = plan(d.nx, d.ny, iters, checking, choices);
+    Scratch scratch(s);
+    IterControl ctl(s, scratch, iters, epsil, P.nblocks, 2);
+    CILREG_TRY(ctl.status());
+    const size_t bytes = sizeof(float) * (size_t)d.n;
+    if (iters <= 0) CILREG_CUDA(cudaMemcpyAsync(u_out, in.f, bytes, cudaMemcpyDeviceToDevice, s));
+    const int nl = count_spans(iters, P.T, checking);
+    // launch k writes U to ub[(nl - 1 - k) & 1] (the last one u_out), B to bb[k & 1]
+    float *ub[2] = {u_out, nullptr}, *bb[2][2] = {};
+    if (nl > 1) ub[1] = scratch.floats(d.n);
+    for (int i = 0; i < 2 && (nl > 1 || warm); i++)
+        for (int c = 0; c < 2; c++) bb[i][c] = scratch.floats(d.n);
+    if (scratch.status() != OK) return scratch.status();
+    Args a = {};
+    a.f = in.f;
+    a.lambda = in.lambda;
+    a.mu = in.mu;
+    a.norm = in.norm;
+    a.dlam = dlam;
+    a.aniso = aniso;
+    CILREG_TRY(run_spans(P, ctl, iters, checking, d, host_aligned8(in.f) && host_aligned8(u_out),
+                         [&](int k, const Span&, const Frame& fr) -> int {
+                             a.first = k == 0;
+                             a.u = k == 0 ? in.f : ub[(nl - k) & 1];
+                             a.un = ub[(nl - 1 - k) & 1];
+                             for (int c = 0; c < 2; c++) {
+                                 a.d0[c] = warm ? warm->dd[c] : nullptr;
+                                 a.bp[c] = k > 0 ? bb[(k + 1) & 1][c] : warm ? warm->bb[c] : nullptr;
+                                 a.bn[c] = (k == nl - 1 && !warm) ? nullptr : bb[k & 1][c];
+                             }
+                             CILREG_CUDA(launch_pdl(pick(P.R, checking), grid_of(P, fr, checking), dim3(32, NW, 1), 0,
+                                                    s, a, fr));
+                             return OK;
+                         }));
+    StopCtl done;
+    CILREG_TRY(ctl.finish(info, &done));
+    const int end = done.stop ? span_of_check(done.iters) : nl - 1;
+    if ((nl - 1 - end) & 1) CILREG_CUDA(cudaMemcpyAsync(u_out, ub[1], bytes, cudaMemcpyDeviceToDevice, s));
+    // a warm run leaves B of the iteration before its last U; the caller
+    // shrinks once more from that U
+    for (int c = 0; c < 2 && warm && iters > 0; c++)
+        CILREG_CUDA(cudaMemcpyAsync(warm->bb[c], bb[end & 1][c], bytes, cudaMemcpyDeviceToDevice, s));
+    return OK;
+}
+
+}  // namespace cilreg

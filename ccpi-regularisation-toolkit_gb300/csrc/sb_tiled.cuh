@@ -2,6 +2,7 @@
 // one 2.5D streaming kernel (sb_tiled.cu).
 #pragma once
 
+#include "drivers.cuh"
 #include "runtime.cuh"
 
 namespace cilreg {
@@ -42,5 +43,13 @@ int sb_sweep2_step(const SbPlan& T, const SbSweepArgs& a, const Dims& d, const S
 // partial slots as sb_sweep2_step)
 int sb_fused_step(const SbPlan& T, const SbFusedArgs& a, bool aniso, const Dims& d, const StopCtl* ctl, int check,
                   double2* partials, cudaStream_t s);
+
+// 2D images run several outer iterations per launch (sb_strip.cu;
+// CILREG_SB_KERNEL or CILREG_STRIP2D=0 keep one per launch).  `in` brings f and
+// the scalars; with `warm`, iteration 0 takes its D and B, and its bb receive
+// B^{n-1} of the n iterations run
+bool sb_strip_applies(const Dims& d);
+int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, int iters, float epsil, const Dims& d,
+                 cudaStream_t s, float* info, SbWarm* warm);
 
 }  // namespace cilreg
