@@ -413,6 +413,7 @@ int tgv_run_fused(const float* f, float* u_out, float lam, float alpha1, float a
 int tgv_run(const float* f, float* u_out, float lam, float alpha1, float alpha0, int iters, float L2, float epsil,
             const Dims& d, cudaStream_t s, float* info) {
     CILREG_RANGE("cilreg TGV");
+    if (tgv_strip_applies(d)) return tgv_strip_run(f, u_out, lam, alpha1, alpha0, iters, L2, epsil, d, s, info);
     const bool three = d.nz > 1;
     const int np = three ? 3 : 2, nq = three ? 6 : 3;
     Scratch scratch(s);

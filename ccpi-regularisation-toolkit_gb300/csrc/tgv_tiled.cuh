@@ -84,4 +84,10 @@ void tgv_primal_tiles(const Dims& d, int& gx, int& gy, int& gz, int& zc);
 int tgv_primal_batch_step(const TgvBatchVol* d_vols, const int* d_ptile_vol, long long nptiles, bool three, int check,
                           cudaStream_t s);
 
+// 2D images run several iterations per launch (tgv_strip.cu; CILREG_TGV_KERNEL
+// or CILREG_STRIP2D=0 keep one per launch)
+bool tgv_strip_applies(const Dims& d);
+int tgv_strip_run(const float* f, float* u_out, float lam, float alpha1, float alpha0, int iters, float L2,
+                  float epsil, const Dims& d, cudaStream_t s, float* info);
+
 }  // namespace cilreg
