@@ -39,13 +39,17 @@ def _forward_one(f, lam, iters, method, nonneg):
     return out
 
 
-def _vjp_one(f, ybar, lam, iters, method, nonneg, ckpt, fbar):
-    lb = ctypes.c_double(0.0)
-    st = cilregcuda.cilreg_fgp_tv_vjp_dev(f.data_ptr(), ybar.data_ptr(), fbar.data_ptr(), ctypes.byref(lb),
-                                          float(lam), int(iters), int(method), int(nonneg), int(ckpt),
-                                          *_dims(tuple(f.shape)), torch.cuda.current_stream(f.device).cuda_stream)
+def _vjp(f, ybar, lams, iters, method, nonneg, ckpt, shape):
+    """(fbar, lambda gradients) of the volumes of `shape` that f holds, all in one native run."""
+    n = len(lams)
+    fbar = torch.empty_like(f)
+    lbars = (ctypes.c_double * n)()
+    st = cilregcuda.cilreg_fgp_tv_vjp_batch_dev(n, f.data_ptr(), ybar.data_ptr(), fbar.data_ptr(), lbars,
+                                                (ctypes.c_float * n)(*lams), int(iters), int(method), int(nonneg),
+                                                int(ckpt), *_dims(shape),
+                                                torch.cuda.current_stream(f.device).cuda_stream)
     check_status(st)
-    return lb.value
+    return fbar, list(lbars)
 
 
 def _parallel(vjp, vols, ybars, lams):
@@ -103,12 +107,8 @@ class FGPTVFunction(torch.autograd.Function):
     def backward(ctx, ybar):
         (f,) = ctx.saved_tensors
         iterations, method, nonneg, ckpt, batched = ctx.cfg
-        ybar = ybar.contiguous()
-        vols = list(f) if batched else [f]
-        ybars = list(ybar) if batched else [ybar]
-        fbars, lbars = _parallel(lambda v, yb, lam, fb: _vjp_one(v, yb, lam, iterations, method, nonneg, ckpt, fb),
-                                 vols, ybars, ctx.lams)
-        fbar = torch.stack(fbars) if batched else fbars[0]
+        fbar, lbars = _vjp(f, ybar.contiguous(), ctx.lams, iterations, method, nonneg, ckpt,
+                           tuple(f.shape[1:] if batched else f.shape))
         if len(ctx.lam_shape) == 0 or (len(lbars) > 1 and int(torch.tensor(ctx.lam_shape).prod()) == 1):
             lam_bar = torch.tensor(sum(lbars), dtype=torch.float64).reshape(ctx.lam_shape)
         else:

@@ -75,6 +75,8 @@ _PP = ctypes.POINTER(ctypes.c_void_p)
 _IP = ctypes.POINTER(ctypes.c_int)
 _VJP_SIGS = {
     "cilreg_fgp_tv_vjp_dev": [_V, _V, _V, ctypes.POINTER(ctypes.c_double), _F, _I, _I, _I, _I, _I, _I, _I, _V],
+    "cilreg_fgp_tv_vjp_batch_dev": [_I, _V, _V, _V, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(_F), _I, _I, _I,
+                                    _I, _I, _I, _I, _V],
     "cilreg_rof_tv_vjp_dev": [_V, _V, _V, ctypes.POINTER(ctypes.c_double), _F, _I, _F, _I, _I, _I, _I, _V],
 }
 _SESSION_SIGS = {

@@ -201,6 +201,12 @@ int cilreg_tgv_batch_dev(int nvol, const float *const *d_in, float *const *d_out
 int cilreg_fgp_tv_vjp_dev(const float *d_in, const float *d_ybar, float *d_inbar, double *lambar, float lambdaPar,
                           int iters, int methodTV, int nonneg, int checkpoint, int dimX, int dimY, int dimZ,
                           void *stream);
+/* The same for nvol volumes of one shape that lie one after another in d_in,
+ * d_ybar and d_inbar, all advanced together; lambar and lambdaPar (host) hold
+ * one value per volume. */
+int cilreg_fgp_tv_vjp_batch_dev(int nvol, const float *d_in, const float *d_ybar, float *d_inbar, double *lambar,
+                                const float *lambdaPar, int iters, int methodTV, int nonneg, int checkpoint, int dimX,
+                                int dimY, int dimZ, void *stream);
 /* The same for the unrolled ROF-TV map y = ROF(f, lambda) with scalar lambda,
  * time step tau and `iters` iterations (the map cilreg_rof_tv_dev computes with
  * d_lambda = NULL and epsil = 0); `checkpoint` >= 1 iterations per segment

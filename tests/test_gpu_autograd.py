@@ -302,3 +302,23 @@ def test_rof_vjp_rejects_bad_arguments():
     assert fn(x.data_ptr(), x.data_ptr(), x.data_ptr(), ctypes.byref(lb), 0.05, 0, 0.01, 5, 6, 5, 4, s) == -2
     assert fn(x.data_ptr(), x.data_ptr(), x.data_ptr(), ctypes.byref(lb), 0.05, 10, 0.01, 0, 6, 5, 4, s) == -2
     assert fn(None, x.data_ptr(), x.data_ptr(), ctypes.byref(lb), 0.05, 10, 0.01, 5, 6, 5, 4, s) == -2
+
+
+@pytest.mark.parametrize("shape", [(1, 5, 7), (3, 29, 33), (70, 13, 57), (29, 25)])
+@pytest.mark.parametrize("iters", [1, 20, 21, 43])
+def test_fgp_vjp_of_a_batch_equals_single_calls(shape, iters):
+    """Volumes of one shape through one native run (tile, chunk and segment edges)."""
+    import torch
+
+    g = torch.Generator("cuda").manual_seed(4)
+    f = torch.rand((3,) + shape, generator=g, device="cuda")
+    ybar = torch.randn(f.shape, generator=g, device="cuda")
+    lams = [0.03, 0.06, 0.1]
+    from ccpi.filters.autograd import _vjp
+
+    fbar, lbar = _vjp(f, ybar, lams, iters, 0, 1, 20, shape)
+    for v in range(3):
+        one, l1 = _vjp(f[v].clone(), ybar[v].clone(), lams[v : v + 1], iters, 0, 1, 20, shape)
+        np.testing.assert_array_equal(fbar[v].cpu().numpy(), one.cpu().numpy())
+        # the same FP32 sums per column of planes, added in FP64 in another order
+        np.testing.assert_allclose(lbar[v], l1[0], rtol=1e-9, atol=1e-9)
