@@ -60,6 +60,25 @@ int use_device(int dev) {
     return OK;
 }
 
+void retain_scratch() {
+    static std::once_flag once[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return;
+    }
+    std::call_once(once[dev], [dev]() {
+        cudaMemPool_t pool;
+        uint64_t thr = 0;
+        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr) == cudaSuccess && thr < (2ULL << 30)) {
+            thr = 2ULL << 30;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
+        }
+        cudaGetLastError();
+    });
+}
+
 int release_cached(int dev) {
     CILREG_TRY(use_device(dev));
     CILREG_CUDA(cudaDeviceSynchronize());

@@ -78,10 +78,17 @@ int resident_ctas(K kernel, int threads) {
     return r;
 }
 
+// Let the current device's pool keep up to 2 GiB of freed scratch (calls on host
+// arrays, use_device, keep all of it).  A pool that keeps none hands its memory
+// back at every synchronisation and maps it anew in the next call: 0.2 ms on a
+// 512^2 image, 1.5 ms on 43 M voxels of scratch.  cilreg_release_cached and a
+// failed allocation give it back.
+void retain_scratch();
+
 // stream-ordered scratch buffers freed when the object is destroyed
 class Scratch {
 public:
-    explicit Scratch(cudaStream_t s) : stream_(s) {}
+    explicit Scratch(cudaStream_t s) : stream_(s) { retain_scratch(); }
     ~Scratch();
     // allocate `count` floats (64-byte aligned); returns nullptr on failure
     float* floats(long long count);
