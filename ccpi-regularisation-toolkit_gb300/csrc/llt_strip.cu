@@ -21,6 +21,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     __shared__ float2 first[2][2][NW][32], last[2][2][NW][32];  // [slot][row from the end]
     const Place<R> q(fr, CHECK, max(tile_index<CHECK>(fr), 0));
     const int lane = q.lane, w = q.w;
+    const bool odd = q.nx & 1;
     const float2 EPS2 = splat(1.0e-12f), MTWO2 = splat(-2.0f);
     const float2 tau2 = splat(tau), lrof2 = splat(lam_rof), mlllt2 = splat(-lam_llt);
     float2 f[R], u[R];
@@ -91,7 +92,11 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
                 const float2 l2h = (EDGE && k == q.bottom) ? l2l : nl2;
                 const float2 dyy = add2(fma2(MTWO2, l2, l2h), l2l);
                 const float2 dv1 = sub2(r1, r1l);
-                const float2 t = sub2(fma2(mlllt2, add2(dxx, dyy), mul2(lrof2, add2(dv1, dv2))), sub2(um, f[k]));
+                const float2 lap = add2(dxx, dyy), div = add2(dv1, dv2);
+                // odd rows round as the one-voxel kernel: the sign terms turn a
+                // last-place difference into 5e-5 of the image in 1000 iterations
+                const float2 g = odd ? fma2(lrof2, div, mul2(mlllt2, lap)) : fma2(mlllt2, lap, mul2(lrof2, div));
+                const float2 t = sub2(g, sub2(um, f[k]));
                 const float2 un = fma2(tau2, t, um);
                 if (CHECK && sum) add_norms(q, k, un, um, pa, pb);
                 u[k] = un;
