@@ -26,7 +26,8 @@
 // A CTA of 16 x ROWS threads holds a 32 x ROWS tile with a two-voxel halo:
 // W on the inner 30 x (ROWS-2) points, the update on the inner 28 x (ROWS-4),
 // whole pairs (threads 1..14 of rows 2..ROWS-3).  Tile x origins are even
-// (x0 = 28 bx - 2).  Needs nx even; arrays off 8-byte alignment run the
+// (x0 = 28 bx - 2).  Odd rows (a last pair whose second voxel is the mirrored
+// one: 1150 -> 788 us per 511^3 iteration against k_d4_stream) and arrays off 8-byte alignment run the
 // 4-byte instantiation.
 #include <stdlib.h>
 
@@ -84,13 +85,15 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     yl = min(max(yl, 0), ROWS - 1);
     yh = min(max(yh, 0), ROWS - 1);
     const int oyl = yl * TW + 2 * tx, oyh = yh * TW + 2 * tx;
-    const int col = min(max(y, 0), ny - 1) * nx + min(max(X, 0), nx - 2);
+    const int col = min(max(y, 0), ny - 1) * nx + (ALIGNED ? min(max(X, 0), nx - 2) : pair_col(X, nx));
+    const int dc = ALIGNED ? 1 : pair_step(X, nx);
+    const bool oend = X + 1 == nx;  // the pair's first voxel ends an odd row
     const int z0 = blockIdx.z * zc;
     const int z1 = min(z0 + zc, nz);
     const int sxy = d.sxy;
     auto ldg2 = [&](const float* p) -> float2 {
         if (ALIGNED) return __ldg(reinterpret_cast<const float2*>(p));
-        return make_float2(__ldg(p), __ldg(p + 1));
+        return make_float2(__ldg(p), __ldg(p + dc));
     };
     auto ld_u = [&](int k) -> float2 { return ldg2(U + (ring_plane(k, nz) * sxy + col)); };
 
@@ -169,7 +172,8 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
         // published in the previous step
         if (FULL) {
             const int kf = j - 2;
-            const Nb w0 = nb(sW[WK], o);
+            Nb w0 = nb(sW[WK], o);
+            if (!ALIGNED && oend) w0.hi.x = w0.lo.x;
             const float2 w = w0.c;
             const float2 lx = fma2(MTWO2, w, add2(w0.lo, w0.hi));
             const float2 ly = fma2(MTWO2, w, add2(ld2(sW[WK] + oyl), ld2(sW[WK] + oyh)));
@@ -185,12 +189,13 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
                     st2(dst, un);
                 } else {
                     dst[0] = un.x;
-                    dst[1] = un.y;
+                    if (!oend) dst[1] = un.y;
                 }
                 if (CHECK) {
-                    const float2 df = sub2(un, u);
-                    pa = fma2(df, df, pa);
-                    pb = fma2(un, un, pb);
+                    const float2 df = sub2(un, u), dm = make_float2(df.x, !ALIGNED && oend ? 0.f : df.y);
+                    const float2 um = make_float2(un.x, !ALIGNED && oend ? 0.f : un.y);
+                    pa = fma2(dm, dm, pa);
+                    pb = fma2(um, um, pb);
                 }
             }
         }
@@ -323,7 +328,7 @@ PairKernel pick2d(bool check, bool aligned) {
 bool d4_pair_applies(const Dims& d) {
     // CILREG_D4_KERNEL=stream (or simple) keeps a one-voxel kernel
     const char* e = getenv("CILREG_D4_KERNEL");
-    return d.nx % 2 == 0 && d.n < (1LL << 31) && !(e && e[0] != '\0' && e[0] != 'p');
+    return pair::pair_rows(d) && !(e && e[0] != '\0' && e[0] != 'p');
 }
 
 D4Plan d4_pair_plan(const Dims& d) {
@@ -351,7 +356,7 @@ D4Plan d4_pair_plan(const Dims& d) {
 
 int d4_pair_step(const D4Plan& T, const float* cur, float* nxt, const float* f, float lam, float tau, float isg2,
                  const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s) {
-    const bool aligned = host_aligned8(cur) && host_aligned8(nxt) && host_aligned8(f);
+    const bool aligned = d.nx % 2 == 0 && host_aligned8(cur) && host_aligned8(nxt) && host_aligned8(f);
     CILREG_CUDA(launch_pdl(d.nz == 1 ? pick2d(check != 0, aligned) : pick(check != 0, aligned), T.grid, T.block, 0,
                            s, cur, nxt, f, lam, tau, isg2, d, T.zchunk, ctl, partials));
     return OK;

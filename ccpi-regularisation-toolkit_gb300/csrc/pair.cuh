@@ -47,6 +47,21 @@ __device__ __forceinline__ float2 rcp2(float2 x) {
     return fma2(r, fma2(neg2(x), r, make_float2(1.0f, 1.0f)), r);
 }
 
+// Rows of odd length (3D): the last pair's second voxel lies beyond the row and
+// holds the mirrored voxel nx-2, so that the first voxel's upper neighbour is
+// the pair's own second voxel as everywhere else.  Column of a pair's first
+// voxel and the step to its second, clamped into the row.
+__device__ __forceinline__ int pair_col(int X, int nx) { return min(max(X, 0), nx - 1); }
+__device__ __forceinline__ int pair_step(int X, int nx) {
+    const int c1 = (X + 1 == nx) ? nx - 2 : min(max(X + 1, 0), nx - 1);
+    return c1 - pair_col(X, nx);
+}
+// the volumes of the 3D two-voxel kernels (8-byte accesses need even rows) and
+// the images of the 2D ones
+inline bool pair_rows(const Dims& d) {
+    return d.n < (1LL << 31) && (d.nx % 2 == 0 || (d.nz > 1 && d.nx >= 3));
+}
+
 // 8-byte access of a pair (shared or global memory, 8-byte aligned)
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }

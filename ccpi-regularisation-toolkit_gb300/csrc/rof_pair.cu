@@ -22,8 +22,8 @@
 //
 // A CTA of 16 x 16 threads holds a 32 x 16 tile with a one-voxel halo; the
 // inner 30 x 14 voxels are updated.  Tile x origins are even (x0 = 30 bx - 2)
-// so that the pairs of a tile are the pairs of the volume; the kernel needs
-// nx even, and 8-byte aligned arrays for its 8-byte accesses (ALIGNED; the
+// so that the pairs of a tile are the pairs of the volume; the 8-byte accesses
+// need nx even and 8-byte aligned arrays (ALIGNED; the
 // other instantiation issues two 4-byte accesses instead).
 #include <stdlib.h>
 
@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     yl = min(max(yl, 0), TH - 1);
     const int oyh = yh * TW + 2 * tx, oyl = yl * TW + 2 * tx;
     // pairs outside the volume load the nearest pair inside it
-    const int col = min(max(y, 0), ny - 1) * nx + min(max(X, 0), nx - 2);
+    const int col = min(max(y, 0), ny - 1) * nx + (ALIGNED ? min(max(X, 0), nx - 2) : pair_col(X, nx));
+    const int dc = ALIGNED ? 1 : pair_step(X, nx);
     const int z0 = blockIdx.z * zc;
     const int z1 = min(z0 + zc, nz);
     const int sxy = d.sxy;
@@ -119,13 +120,13 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
             cp_async8(dst, src);
         } else {
             cp_async4(dst, src);
-            cp_async4(dst + 1, src + 1);
+            cp_async4(dst + 1, src + dc);
         }
         cp_async_commit();
     };
     auto ldg2 = [&](const float* p) -> float2 {
         if (ALIGNED) return __ldg(reinterpret_cast<const float2*>(p));
-        return make_float2(__ldg(p), __ldg(p + 1));
+        return make_float2(__ldg(p), __ldg(p + dc));
     };
     float2 pa = splat(0.f), pb = splat(0.f);
     for (int k = z0 - 2; k < z0 + AHEAD; k++) issue(k - z0 + 2, k);
@@ -327,7 +328,7 @@ bool smem_ready() {
 bool rof_pair_applies(const Dims& d) {
     // CILREG_ROF_KERNEL=async (or reg, simple) keeps the one-voxel kernels
     const char* ek = getenv("CILREG_ROF_KERNEL");
-    return d.nx % 2 == 0 && d.n < (1LL << 31) && !(ek && ek[0] != '\0' && ek[0] != 'p');
+    return pair::pair_rows(d) && !(ek && ek[0] != '\0' && ek[0] != 'p');
 }
 
 RofPlan rof_pair_plan(const Dims& d) {
@@ -357,7 +358,7 @@ int rof_pair_step(const RofPlan& T, const float* cur, float* nxt, const float* f
                   float tau, const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s) {
     const bool larr = lam_arr != nullptr;
     const bool aligned =
-        host_aligned8(cur) && host_aligned8(nxt) && host_aligned8(f) && (!larr || host_aligned8(lam_arr));
+        d.nx % 2 == 0 && host_aligned8(cur) && host_aligned8(nxt) && host_aligned8(f) && (!larr || host_aligned8(lam_arr));
     if (d.nz == 1) {
         CILREG_CUDA(launch_pdl(pick2d(check != 0, larr, aligned), T.grid, T.block, 0, s, cur, nxt, f, lam_arr, lam,
                                tau, d, 1, ctl, partials));

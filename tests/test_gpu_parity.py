@@ -726,3 +726,28 @@ def test_fgp_two_voxel_kernel_with_arrays_off_8_byte_alignment():
     (a, ia), (b, ib) = outs
     assert int(ia[0]) == int(ib[0])
     np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 3), (5, 16, 29), (9, 30, 31), (7, 15, 61), (70, 29, 57), (3, 1, 5)])
+@pytest.mark.parametrize("alg", ["rof", "d4"])
+def test_odd_rows_of_the_two_voxel_kernels_match_the_one_voxel_kernels(alg, shape, monkeypatch):
+    """3D volumes with rows of odd length: the last pair's second voxel is the
+    mirrored one (tile edges, chunk edges, one row, both stopping variants)."""
+    import torch
+    from ccpi.filters import regularisersCuPy as R
+
+    rng = np.random.default_rng(6)
+    x = torch.from_numpy((rng.random(shape) + np.arange(shape[-1]) // 5 % 2).astype(np.float32)).cuda()
+    name = {"rof": "CILREG_ROF_KERNEL", "d4": "CILREG_D4_KERNEL"}[alg]
+
+    def run(tol):
+        if alg == "rof":
+            return R.ROF_TV(x, 0.02, 12, 0.001, tolerance_param=tol).cpu().numpy()
+        return R.Diff4th(x, 0.8, 0.02, 12, 1e-4, tol).cpu().numpy()
+
+    for tol in (0.0, 1e-7):
+        got = run(tol)
+        monkeypatch.setenv(name, {"rof": "async", "d4": "stream"}[alg])
+        want = run(tol)
+        monkeypatch.delenv(name)
+        np.testing.assert_allclose(got, want, rtol=0, atol=1e-5 * float(np.ptp(want)))
