@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
               float tau, float isg2, Dims d, int zc, const StopCtl* ctl, double2* partials) {
     constexpr int TP = Geo<ROWS>::TP, NTP = Geo<ROWS>::NTP;
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     __shared__ __align__(16) float sU[4][TP];
     __shared__ __align__(16) float sW[2][TP];
     if (ctl->stop) return;
@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     if (j <= z1 + 1) step(Ic<3>{}, T_{}, F_{}, j);
     if (j + 1 <= z1 + 1) step(Ic<0>{}, T_{}, F_{}, j + 1);
     if (j + 2 <= z1 + 1) step(Ic<1>{}, T_{}, F_{}, j + 2);
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NTP>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
 }
 

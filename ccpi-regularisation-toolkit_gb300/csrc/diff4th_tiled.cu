@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(NT, 2) k_d4_stream(const float* __restrict__ U
                                                      const float* __restrict__ F, float lam, float tau, float isg2,
                                                      Dims d, int zc, const StopCtl* ctl, double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     __shared__ float sU[4][BY][BX];
     __shared__ float sW[2][BY][BX];
     if (ctl->stop) return;
@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(NT, 2) k_d4_stream(const float* __restrict__ U
     if (j <= z1 + 1) step(Ic<0>{}, std::false_type{}, j);
     if (j + 1 <= z1 + 1) step(Ic<1>{}, std::false_type{}, j + 1);
     if (j + 2 <= z1 + 1) step(Ic<2>{}, std::false_type{}, j + 2);
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 

@@ -211,10 +211,11 @@ template <bool THREE, bool CHECK, typename IT, bool DTV = false>
 __global__ void __launch_bounds__(NT, DTV ? 2 : 3) k_fgp_stream(TiledArgs a, Dims d, int zc, const StopCtl* ctl,
                                                                 double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     if (ctl->stop) return;
     float pa = 0.f, pb = 0.f;
     fgp_stream_tile<THREE, CHECK, IT, DTV>(a, d, zc, blockIdx.x, blockIdx.y, blockIdx.z, pa, pb);
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 

@@ -186,10 +186,11 @@ template <bool CHECK, bool ALIGNED>
 __global__ void __launch_bounds__(NTP, 4) k_fgp_x2(X2Args a, Dims d, int zc, const StopCtl* ctl,
                                                    double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     if (ctl->stop) return;
     float pa = 0.f, pb = 0.f;
     x2_tile<CHECK, ALIGNED>(a, d, zc, blockIdx.x, blockIdx.y, blockIdx.z, pa, pb);
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NTP>(pa, pb, partials, block_slot());
 }
 

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(NTP, MINB)
     k_llt_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam_rof,
                float lam_llt, float tau, Dims d, int zc, const StopCtl* ctl, double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     __shared__ __align__(16) float sU[4][TP];
     __shared__ __align__(16) float sR1[2][TP];  // ROF D1 (j axis), read at j-1
     __shared__ __align__(16) float sR2[2][TP];  // ROF D2 (i axis), read at i-1
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(NTP, MINB)
     if (j <= z1 + 1) step(Ic<3>{}, T_{}, F_{}, j);
     if (j + 1 <= z1 + 1) step(Ic<0>{}, T_{}, F_{}, j + 1);
     if (j + 2 <= z1 + 1) step(Ic<1>{}, T_{}, F_{}, j + 2);
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NTP>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
 }
 

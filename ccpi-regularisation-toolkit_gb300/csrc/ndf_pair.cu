@@ -49,7 +49,6 @@ __global__ void __launch_bounds__(NTP, 4)
     k_ndf_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F, float lam, float sg,
                float isg, float tau, Dims d, int zc, const StopCtl* ctl, double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
     extern __shared__ __align__(16) float smem[];
     float* const ring = smem;
     float* const sFx = ring + RING * TP;
@@ -170,6 +169,7 @@ __global__ void __launch_bounds__(NTP, 4)
     }
     for (; j <= z1 + 1; j++) step(j - z0, T_{}, F_{}, j);
     cp_async_wait<0>();
+    pdl_trigger();
     if (CHECK) block_pair_partial<NTP>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
 }
 

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(NT, 3) k_ndf_stream(const float* __restrict__ 
     __shared__ float sFx[2][BY * BX];
     __shared__ float sFy[2][BY * BX];
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     if (ctl->stop) return;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(NT, 3) k_ndf_stream(const float* __restrict__ 
         }
         if (j <= z1 + 1) step(Ic<0>{}, std::true_type{}, j);
     }
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(NT, 3) k_pd_stream(PdStreamArgs a, Dims d, int
     __shared__ float sP1[2][BY][BX];
     __shared__ float sP2[2][BY][BX];
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     if (ctl->stop) return;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(NT, 3) k_pd_stream(PdStreamArgs a, Dims d, int
         q3 = nq3;
         fq = nf;
     }
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 

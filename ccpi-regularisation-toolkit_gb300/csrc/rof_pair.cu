@@ -71,14 +71,14 @@ __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
-template <bool CHECK, bool LARR, bool ALIGNED, int ROWS>
+template <bool CHECK, bool LARR, bool ALIGNED, int ROWS, bool LATE>
 __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     k_rof_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F,
                const float* __restrict__ lam_arr, float lam, float tau, Dims d, int zc, const StopCtl* ctl,
                double2* partials) {
     constexpr int TH = Geo<ROWS>::TH, OYP = Geo<ROWS>::OYP, NTP = Geo<ROWS>::NTP, TP = Geo<ROWS>::TP;
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (!LATE) pdl_trigger();
     extern __shared__ __align__(16) float smem[];
     float* const ring = smem;
     float* const sD1 = ring + RING * TP;
@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     }
     for (; j <= z1 + 1; j++) step(j - z0, T_{}, F_{}, j);
     cp_async_wait<0>();
+    if (LATE) pdl_trigger();
     if (CHECK) block_pair_partial<NTP>(pa.x + pa.y, pb.x + pb.y, partials, block_slot());
 }
 
@@ -290,14 +291,22 @@ __global__ void __launch_bounds__(NTP2, 8)
 // A 32-row tile has 7% fewer halo voxels but two CTAs per SM, and measured
 // 0.475 against 0.436 ms per 512^3 iteration.
 constexpr int ROWS = 16;
-using PairKernel = decltype(&k_rof_pair<false, false, true, ROWS>);
+using PairKernel = decltype(&k_rof_pair<false, false, true, ROWS, true>);
 
-PairKernel pick(bool check, bool larr, bool aligned) {
+template <bool LATE>
+PairKernel pick_t(bool check, bool larr, bool aligned) {
     if (aligned)
-        return check ? (larr ? k_rof_pair<true, true, true, ROWS> : k_rof_pair<true, false, true, ROWS>)
-                     : (larr ? k_rof_pair<false, true, true, ROWS> : k_rof_pair<false, false, true, ROWS>);
-    return check ? (larr ? k_rof_pair<true, true, false, ROWS> : k_rof_pair<true, false, false, ROWS>)
-                 : (larr ? k_rof_pair<false, true, false, ROWS> : k_rof_pair<false, false, false, ROWS>);
+        return check ? (larr ? k_rof_pair<true, true, true, ROWS, LATE> : k_rof_pair<true, false, true, ROWS, LATE>)
+                     : (larr ? k_rof_pair<false, true, true, ROWS, LATE> : k_rof_pair<false, false, true, ROWS, LATE>);
+    return check ? (larr ? k_rof_pair<true, true, false, ROWS, LATE> : k_rof_pair<true, false, false, ROWS, LATE>)
+                 : (larr ? k_rof_pair<false, true, false, ROWS, LATE> : k_rof_pair<false, false, false, ROWS, LATE>);
+}
+// late: where the kernel triggers its successor (pdl_many_waves), chosen here
+// at compile time (the late trigger's code costs the early variant 2%): late
+// for a grid of one wave, four CTAs per SM (192^3 32.8 -> 31.0 us per
+// iteration), early above (256^3 62.8 against 63.6)
+PairKernel pick(bool check, bool larr, bool aligned, bool late) {
+    return late ? pick_t<true>(check, larr, aligned) : pick_t<false>(check, larr, aligned);
 }
 
 PairKernel pick2d(bool check, bool larr, bool aligned) {
@@ -314,8 +323,8 @@ bool smem_ready() {
         bool r = true;
         for (int c = 0; c < 2; c++)
             for (int l = 0; l < 2; l++)
-                for (int a = 0; a < 2; a++)
-                    r = r && cudaFuncSetAttribute(pick(c, l, a), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                for (int a = 0; a < 4; a++)
+                    r = r && cudaFuncSetAttribute(pick(c, l, a & 1, a & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)Geo<ROWS>::SMEM) == cudaSuccess;
         cudaGetLastError();
         return r;
@@ -345,7 +354,7 @@ RofPlan rof_pair_plan(const Dims& d) {
     const int gx = tiles_x(d.nx), gy = (d.ny + Geo<ROWS>::OYP - 1) / Geo<ROWS>::OYP;
     int resident = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &resident, k_rof_pair<false, false, true, ROWS>, Geo<ROWS>::NTP, Geo<ROWS>::SMEM);
+        &resident, k_rof_pair<false, false, true, ROWS, false>, Geo<ROWS>::NTP, Geo<ROWS>::SMEM);
     if (e != cudaSuccess || resident <= 0) resident = 1;
     cudaGetLastError();
     T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
@@ -366,7 +375,7 @@ int rof_pair_step(const RofPlan& T, const float* cur, float* nxt, const float* f
     }
     if (!smem_ready())
         return fail(ERR_CUDA, __FILE__, __LINE__, "cannot raise the shared-memory limit of k_rof_pair");
-    CILREG_CUDA(launch_pdl(pick(check != 0, larr, aligned), T.grid, T.block, Geo<ROWS>::SMEM, s, cur, nxt, f,
+    CILREG_CUDA(launch_pdl(pick(check != 0, larr, aligned, T.nblocks <= 4LL * sm_count()), T.grid, T.block, Geo<ROWS>::SMEM, s, cur, nxt, f,
                            lam_arr, lam, tau, d, T.zchunk, ctl, partials));
     return OK;
 }

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(NT, 3) k_rof_stream(const float* __restrict__ 
         lv0 = (LARR && o_pt) ? __ldg(lam_arr + col) : lam;
     }
     pdl_wait();  // the previous iteration has completed and its writes are visible
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     if (ctl->stop) return;
 
     if constexpr (!THREE) {
@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(NT, 3) k_rof_stream(const float* __restrict__ 
         }
         if (j <= z1 + 1) step(Ic<0>{}, std::true_type{}, j);
     }
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(NT, 3) k_rof_async(const float* __restrict__ U
                                                      float lam, float tau, Dims d, int zc, const StopCtl* ctl,
                                                      double2* partials) {
     pdl_wait();  // the previous iteration has completed (launch_pdl)
-    pdl_trigger();
+    if (pdl_many_waves()) pdl_trigger();
     __shared__ float sU[RING][BY * BX];
     __shared__ float sD1[2][BY * BX];
     __shared__ float sD2[2][BY * BX];
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(NT, 3) k_rof_async(const float* __restrict__ U
     }
     for (; j <= z1 + 1; j++) step(j - z0, std::true_type{}, j);
     cp_async_wait<0>();
+    if (!pdl_many_waves()) pdl_trigger();
     if (CHECK) block_pair_partial<NT>(pa, pb, partials, block_slot());
 }
 

@@ -190,6 +190,20 @@ int run_replayed(int iters, int G, cudaStream_t s, Enq enqueue, Tail tail = Tail
 // status and clears it from the thread's error state.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// Where a streaming kernel triggers.  At its start, the next grid's CTAs take
+// the slots that this grid leaves free and wait in them, unevenly: the SMs
+// with fewest of this grid's CTAs get most of the next's, and a grid of one or
+// two CTAs per SM then runs three or four on some (ROF 96^3 14.2 us per
+// iteration; 11.8 with the trigger after a CTA's last plane).  A grid of many
+// waves leaves no free slots and gains from the early start (ROF 512^3 436
+// against 448 us).
+// Read anew at each use (volatile): held in a register over the plane loop, the
+// answer cost D4's kernel 5%.
+__device__ __forceinline__ bool pdl_many_waves() {
+    unsigned x, y, z;
+    asm volatile("mov.u32 %0, %%nctaid.x;\n\tmov.u32 %1, %%nctaid.y;\n\tmov.u32 %2, %%nctaid.z;" : "=r"(x), "=r"(y), "=r"(z));
+    return x * y * z >= 4096u;
+}
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
