@@ -349,7 +349,7 @@ D4Plan d4_pair_plan(const Dims& d) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_d4_pair<false, true, ROWS>, Geo<ROWS>::NTP, 0);
     if (e != cudaSuccess || resident <= 0) resident = 1;
     cudaGetLastError();
-    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
+    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 3, ZCHUNK, 1.25, 1e9);
     T.grid = dim3(gx, gy, (d.nz + T.zchunk - 1) / T.zchunk);
     T.nblocks = (long long)T.grid.x * T.grid.y * T.grid.z;
     return T;

@@ -194,7 +194,7 @@ D4Plan d4_stream_plan(const Dims& d) {
     if (d.nz > 1) {
         static const int resident = resident_ctas(k_d4_stream<true, false, int>, NT);
         const long long tiles = (long long)((d.nx + OX - 1) / OX) * ((d.ny + OY - 1) / OY);
-        T.zchunk = wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK);
+        T.zchunk = wave_zchunk(tiles, d.nz, resident, 3, ZCHUNK, 1.25, 1e9);
     } else {
         T.zchunk = 1;
     }

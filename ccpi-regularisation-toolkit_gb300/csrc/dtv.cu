@@ -63,7 +63,7 @@ int dtv_run(const float* f, const float* ref, float* u_out, float lam, int iters
     Scratch scratch(s);
     // 2D images with an even row length: the two-pixel kernel; otherwise the
     // streaming kernel (whatever CILREG_FGP_KERNEL says, bar 'stream')
-    TiledPlan T = fgp_tiled_plan(d);
+    TiledPlan T = fgp_tiled_plan(d, 2);  // two CTAs of the dTV instantiation per SM
     if (d.nz == 1) {
         const TiledPlan X = fgp_x2_plan(d);
         if (X.use) T = X;

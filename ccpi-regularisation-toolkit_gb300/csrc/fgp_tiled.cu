@@ -475,7 +475,8 @@ TiledPlan fgp_tiled_plan(const Dims& d, int resident_ctas_per_sm) {
         // many volumes and keeps fgp_default_zchunk)
         static const int resident = resident_ctas(k_fgp_stream<true, false, int>, NT);
         const long long tiles = (long long)((d.nx + OX - 1) / OX) * ((d.ny + OY - 1) / OY);
-        T.zchunk = wave_zchunk(tiles, d.nz, resident_ctas_per_sm > 0 ? resident_ctas_per_sm : resident, 2, ZCHUNK);
+        T.zchunk = resident_ctas_per_sm > 0 ? wave_zchunk(tiles, d.nz, resident_ctas_per_sm, 2, ZCHUNK)
+                                            : wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK, 2.5);
     } else {
         T.zchunk = 1;
     }

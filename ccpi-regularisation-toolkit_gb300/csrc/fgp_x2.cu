@@ -431,7 +431,7 @@ TiledPlan fgp_x2_plan(const Dims& d) {
     T.block = dim3(PX, ROWS, 1);
     static const int resident = resident_ctas(k_fgp_x2<false, true>, NTP);
     const int gx = tiles_x(d.nx), gy = (d.ny + OYP - 1) / OYP;
-    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
+    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK, 2.5);
     T.grid = dim3(gx, gy, (d.nz + T.zchunk - 1) / T.zchunk);
     T.nblocks = (long long)T.grid.x * T.grid.y * T.grid.z;
     return T;

@@ -202,7 +202,7 @@ LltPlan llt_plan(const Dims& d) {
     if (d.nz > 1) {
         static const int resident = resident_ctas(k_llt_stream<true, false, int>, NT);
         const long long tiles = (long long)((d.nx + OX - 1) / OX) * ((d.ny + OY - 1) / OY);
-        T.zchunk = wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK);
+        T.zchunk = wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK, 1.25);
     } else {
         T.zchunk = 1;
     }

@@ -329,7 +329,7 @@ LltPlan llt_pair_plan(const Dims& d) {
     T.block = dim3(PX, ROWS, 1);
     const int gx = (d.nx + OX4 - 1) / OX4, gy = (d.ny + OY4 - 1) / OY4;
     static const int resident = resident_ctas(pick(false, true), NTP);
-    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
+    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK, 2.5);
     T.grid = dim3(gx, gy, (d.nz + T.zchunk - 1) / T.zchunk);
     T.nblocks = (long long)T.grid.x * T.grid.y * T.grid.z;
     return T;

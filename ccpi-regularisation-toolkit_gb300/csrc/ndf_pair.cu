@@ -292,7 +292,12 @@ bool smem_ready() {
 bool ndf_pair_applies(const Dims& d) {
     // CILREG_NDF_KERNEL=stream (or simple) keeps a one-voxel kernel
     const char* e = getenv("CILREG_NDF_KERNEL");
-    return d.nx % 2 == 0 && d.n < (1LL << 31) && !(e && e[0] != '\0' && e[0] != 'p');
+    if (e && e[0] != '\0') return pair::pair_rows(d) && d.nx % 2 == 0 && e[0] == 'p';
+    // volumes from 2^24 voxels: below, k_ndf_stream's two planes of look-ahead
+    // and three CTAs of 16 warps per SM are faster (96^3 7.0 against 10.7 us
+    // per iteration, 128^3 10.0 against 12.2, 192^3 25.4 against 27.5; 256^3
+    // 56.0 against 55.6, 512^3 418 against 388); the same bits
+    return d.nx % 2 == 0 && d.n < (1LL << 31) && (d.nz == 1 || d.n >= (1LL << 24));
 }
 
 NdfPlan ndf_pair_plan(const Dims& d) {
@@ -314,7 +319,7 @@ NdfPlan ndf_pair_plan(const Dims& d) {
         resident <= 0)
         resident = 1;
     cudaGetLastError();
-    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
+    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK, 1.25);
     T.grid = dim3(gx, gy, (d.nz + T.zchunk - 1) / T.zchunk);
     T.nblocks = (long long)T.grid.x * T.grid.y * T.grid.z;
     return T;

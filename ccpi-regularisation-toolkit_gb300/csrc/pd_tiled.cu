@@ -213,7 +213,7 @@ PdPlan pd_stream_plan(const Dims& d) {
     if (d.nz > 1) {
         static const int resident = resident_ctas(k_pd_stream<true, false, int>, NT);
         const long long tiles = (long long)((d.nx + OX - 1) / OX) * ((d.ny + OY - 1) / OY);
-        T.zchunk = wave_zchunk(tiles, d.nz, resident, 1, ZCHUNK);
+        T.zchunk = wave_zchunk(tiles, d.nz, resident, 1, ZCHUNK, 2.5);
     } else {
         T.zchunk = 1;
     }

@@ -357,7 +357,7 @@ RofPlan rof_pair_plan(const Dims& d) {
         &resident, k_rof_pair<false, false, true, ROWS, false>, Geo<ROWS>::NTP, Geo<ROWS>::SMEM);
     if (e != cudaSuccess || resident <= 0) resident = 1;
     cudaGetLastError();
-    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK);
+    T.zchunk = wave_zchunk((long long)gx * gy, d.nz, resident, 2, ZCHUNK, 1.25);
     T.grid = dim3(gx, gy, (d.nz + T.zchunk - 1) / T.zchunk);
     T.nblocks = (long long)T.grid.x * T.grid.y * T.grid.z;
     return T;

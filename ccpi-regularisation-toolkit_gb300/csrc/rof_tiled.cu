@@ -497,7 +497,7 @@ RofPlan rof_tiled_plan(const Dims& d) {
     if (d.nz > 1) {
         // CTAs per SM of the 3D kernel (every variant has the same register cap)
         static const int resident = resident_ctas(k_rof_stream<true, false, false, int>, NT);
-        T.zchunk = wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK);
+        T.zchunk = wave_zchunk(tiles, d.nz, resident, 2, ZCHUNK, 1.25);
     } else {
         T.zchunk = 1;
     }

@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -120,7 +121,8 @@ bool pdl_enabled() {
     return !(e && e[0] == '0');
 }
 
-int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chunk) {
+int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chunk, double busy,
+                double waves) {
     if (nz <= 1) return 1;
     if (max_chunk > nz) max_chunk = nz;
     if (const char* e = getenv("CILREG_STREAM_ZCHUNK")) {
@@ -130,10 +132,15 @@ int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chu
     const long long slots = (long long)sm_count() * (resident > 0 ? resident : 1);
     int best = max_chunk;
     double best_cost = -1.0;
-    for (int zc = max_chunk; zc >= 8 || zc == max_chunk; zc--) {
+    const long long sms = sm_count();
+    if ((double)(tiles_xy * ((nz + 7) / 8)) > waves * (double)slots) busy = 0.0;
+    if (busy > 0.0) extra++;
+    for (int zc = max_chunk; zc >= (busy > 0.0 ? 4 : 8) || zc == max_chunk; zc--) {
         const long long blocks = tiles_xy * ((nz + zc - 1) / zc);
         const long long rounds = (blocks + slots - 1) / slots;
-        const double cost = (double)rounds * (double)(zc + extra);
+        double share = (double)rounds;
+        if (busy > 0.0) share = std::max(busy, (double)((blocks + sms - 1) / sms));
+        const double cost = share * (double)(zc + extra);
         if (best_cost < 0 || cost < best_cost * 0.995) {  // prefer longer chunks on ties
             best_cost = cost;
             best = zc;

@@ -65,9 +65,19 @@ cudaStream_t thread_stream(int dev);
 int sm_count();
 
 // z-chunk length for a 2.5D streaming kernel: `tiles_xy` CTAs per z chunk,
-// `resident` CTAs per SM, `extra` pipeline steps per chunk besides its planes.
-// Minimises (rounds of CTAs over the SMs) x (steps per CTA), up to `max_chunk`.
-int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chunk);
+// `resident` CTAs per SM, `extra` pipeline steps per chunk besides its planes,
+// up to `max_chunk` planes.  Minimises (steps per CTA) x (time of a step):
+//   busy > 0, and chunks of 8 planes make at most `waves` waves of CTAs: a step
+//     takes as long as the CTAs that share an SM, at least `busy` of them
+//     (below that, latency), need to issue it: max(busy, ceil(CTAs / SMs)).
+//     Of chunks from 4 to 64 planes on nine volumes from 64^3 to 256^3 this
+//     picks one within 1.3-4% of the fastest (ROF, NDF, Diff4th, LLT-ROF, FGP,
+//     PD; with the late trigger 96^3 ROF 13.8 -> 9.7, FGP 12.7 -> 10.1 us).
+//   otherwise: rounds of CTAs over the SMs' slots.  Above two waves the first
+//     model costs up to 14% (FGP 256^3 133 against 115 us), Diff4th alone
+//     gains from it throughout (512^3 704 -> 680 us).
+int wave_zchunk(long long tiles_xy, int nz, int resident, int extra, int max_chunk, double busy = 0.0,
+                double waves = 2.0);
 
 // CTAs of `kernel` resident per SM at `threads` threads and no dynamic shared
 // memory (at least 1)
