@@ -216,7 +216,7 @@ LltPlan llt_plan(const Dims& d) {
 int llt_run(const float* f, float* u_out, float lam_rof, float lam_llt, int iters, float tau, float epsil,
             const Dims& d, cudaStream_t s, float* info) {
     CILREG_RANGE("cilreg LLT-ROF");
-    if (llt_strip_applies(d)) return llt_strip_run(f, u_out, lam_rof, lam_llt, iters, tau, epsil, d, s, info);
+    if (llt_strip_applies(d, epsil != 0.0f)) return llt_strip_run(f, u_out, lam_rof, lam_llt, iters, tau, epsil, d, s, info);
     Scratch scratch(s);
     const LltPlan T = llt_plan(d);
     IterControl ctl(s, scratch, iters, epsil, T.nblocks);

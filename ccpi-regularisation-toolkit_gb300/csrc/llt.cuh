@@ -37,6 +37,34 @@ __device__ __forceinline__ float2 llt_quot2(float2 v) {
 }
 
 
+// The terms of N second differences.  Where all of them are finite and at least
+// 2^-15 (one test for all: their smallest magnitude, and the sum of the
+// magnitudes, which is not finite where one of them is not), they are sign
+// copies; else each is looked at by itself, as above.
+template <int N>
+__device__ __forceinline__ void llt_terms(const float2 (&v)[N], float2 (&t)[N]) {
+    float least = fminf(fabsf(v[0].x), fabsf(v[0].y)), all = fabsf(v[0].x) + fabsf(v[0].y);
+#pragma unroll
+    for (int i = 1; i < N; i++) {
+        least = fminf(least, fminf(fabsf(v[i].x), fabsf(v[i].y)));
+        all += fabsf(v[i].x) + fabsf(v[i].y);
+    }
+    if (least >= 0x1p-15f && all <= 3.4028234664e38f) {
+#pragma unroll
+        for (int i = 0; i < N; i++) t[i] = make_float2(copysignf(1.0f, v[i].x), copysignf(1.0f, v[i].y));
+        return;
+    }
+    bool divide = false;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        t[i] = llt_sign2(v[i]);
+        divide |= llt_divides2(v[i]);
+    }
+    if (divide)
+#pragma unroll
+        for (int i = 0; i < N; i++) t[i] = llt_quot2(v[i]);
+}
+
 struct LltPlan {
     dim3 grid, block;
     long long nblocks = 0;
@@ -54,7 +82,7 @@ cudaError_t llt_pair_launch(const LltPlan& T, const float* cur, float* nxt, cons
 
 // 2D images run several iterations per launch (llt_strip.cu; CILREG_LLT_KERNEL
 // or CILREG_STRIP2D=0 keep one per launch)
-bool llt_strip_applies(const Dims& d);
+bool llt_strip_applies(const Dims& d, bool checking);
 int llt_strip_run(const float* f, float* u_out, float lam_rof, float lam_llt, int iters, float tau, float epsil,
                   const Dims& d, cudaStream_t s, float* info);
 

@@ -120,22 +120,18 @@ __global__ void __launch_bounds__(NTP, MINB)
             const float2 v3 = add2(fma2(MTWO2, c, uhi), ulo);
             const float2 v1 = add2(fma2(MTWO2, c, ch), cl);
             const float2 v2 = add2(fma2(MTWO2, c, uyh), uyl);
-            float2 t3 = llt_sign2(v3), t1 = llt_sign2(v1), t2 = llt_sign2(v2);
-            if (llt_divides2(v3) | llt_divides2(v1) | llt_divides2(v2)) {
-                t3 = llt_quot2(v3);
-                t1 = llt_quot2(v1);
-                t2 = llt_quot2(v2);
-            }
+            float2 t[3];
+            llt_terms({v1, v2, v3}, t);
             l3c = l3b;
             l3b = l3a;
-            l3a = t3;
+            l3a = t[2];
             r3c = r3b;
             r3b = r3a;
             r3a = n3;
             st2(sR1[WM] + o, n1);
             st2(sR2[WM] + o, n2);
-            st2(sL1[WM] + o, t1);
-            st2(sL2[WM] + o, t2);
+            st2(sL1[WM] + o, t[0]);
+            st2(sL2[WM] + o, t[1]);
         }
         // C. update plane kf = j-2 (LLT_ROF_core.c:404-436); its terms were
         // published in the previous step
