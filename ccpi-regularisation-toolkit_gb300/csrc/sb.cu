@@ -5,6 +5,8 @@
 // grad U + B into D and the Bregman update of B.  Kernels:
 //   k_sb_sweep2  both sweeps of the first outer iteration in one streaming
 //                pass (sb_tiled.cu)
+//   k_sb_pair    every later outer iteration of a 3D volume: as k_sb_fused,
+//                two voxels per thread (sb_pair.cu)
 //   k_sb_fused   every later outer iteration in one streaming pass: D and B
 //                formed from U and the previous B, both sweeps, new U and B
 //                written (sb_tiled.cu); D is never stored
@@ -171,8 +173,11 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
     }
     Scratch scratch(s);
     const SbPlan T = sb_sweep2_plan(d);
+    bool aligned = ((uintptr_t)f | (uintptr_t)u_out) % 8 == 0;
+    for (int c = 0; c < nc && warm; c++) aligned = aligned && (uintptr_t)warm->bb[c] % 8 == 0;
+    const SbPlan T2 = sb_pair_plan(d, aligned);  // of the iterations k >= 1
     const long long nparts = T.use ? T.nblocks : num_blocks(L);
-    IterControl ctl(s, scratch, iters, epsil, nparts);
+    IterControl ctl(s, scratch, iters, epsil, T2.use ? std::max(nparts, T2.nblocks) : nparts);
     CILREG_TRY(ctl.status());
     float* u1 = scratch.floats(d.n);
     if (!u1) return scratch.status();
@@ -232,6 +237,10 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
         z.mu = a.mu;
         z.norm = a.norm;
         z.dlam = a.dlam;
+        auto later_step = [&](int check, cudaStream_t st) {
+            return T2.use ? sb_pair_step(T2, z, a.aniso != 0, d, ctl.ctl(), check, ctl.partials(), st)
+                          : sb_fused_step(T, z, a.aniso != 0, d, ctl.ctl(), check, ctl.partials(), st);
+        };
         if (!ctl.checking() && d.n <= (1LL << 22) && iters > 1) {
             // small volume, fixed count: iteration 0 alone, iterations 1.. as
             // a replayed graph (their launches depend on the parity only)
@@ -247,7 +256,7 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
                     z.bp[c] = bbuf[(i - 1) & 1][c];
                     z.bn[c] = bbuf[i & 1][c];
                 }
-                CILREG_TRY(sb_fused_step(T, z, a.aniso != 0, d, ctl.ctl(), 0, ctl.partials(), st));
+                CILREG_TRY(later_step(0, st));
                 note_launch();
                 return OK;
             }));
@@ -266,11 +275,11 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
                     z.bp[c] = bbuf[(it - 1) & 1][c];
                     z.bn[c] = bbuf[it & 1][c];
                 }
-                CILREG_TRY(sb_fused_step(T, z, a.aniso != 0, d, ctl.ctl(), check, ctl.partials(), s));
+                CILREG_TRY(later_step(check, s));
             }
             note_launch();
             if (check) {
-                CILREG_TRY(ctl.after_check(it, nparts));
+                CILREG_TRY(ctl.after_check(it, (it > 0 && T2.use) ? T2.nblocks : nparts));
                 if (ctl.host_should_stop()) break;
             }
         }

@@ -32,6 +32,7 @@ struct SbPlan {
     long long nblocks = 0;
     int zchunk = 0;
     bool use = false;  // false: the per-sweep kernels of sb.cu run instead
+    bool aligned = false;  // sb_pair_plan: every array is 8-byte aligned
 };
 
 SbPlan sb_sweep2_plan(const Dims& d);
@@ -43,6 +44,13 @@ int sb_sweep2_step(const SbPlan& T, const SbSweepArgs& a, const Dims& d, const S
 // partial slots as sb_sweep2_step)
 int sb_fused_step(const SbPlan& T, const SbFusedArgs& a, bool aniso, const Dims& d, const StopCtl* ctl, int check,
                   double2* partials, cudaStream_t s);
+
+// one outer iteration k >= 1 of a 3D volume with two voxels per thread
+// (sb_pair.cu); its plan's `use` is false where k_sb_fused runs instead.
+// `aligned`: the caller's arrays (f, U, a session's B) are 8-byte aligned
+SbPlan sb_pair_plan(const Dims& d, bool aligned);
+int sb_pair_step(const SbPlan& T, const SbFusedArgs& a, bool aniso, const Dims& d, const StopCtl* ctl, int check,
+                 double2* partials, cudaStream_t s);
 
 // 2D images run several outer iterations per launch (sb_strip.cu;
 // CILREG_SB_KERNEL or CILREG_STRIP2D=0 keep one per launch).  `in` brings f and

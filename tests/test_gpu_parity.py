@@ -751,3 +751,25 @@ def test_odd_rows_of_the_two_voxel_kernels_match_the_one_voxel_kernels(alg, shap
         want = run(tol)
         monkeypatch.delenv(name)
         np.testing.assert_allclose(got, want, rtol=0, atol=1e-5 * float(np.ptp(want)))
+
+
+@pytest.mark.parametrize("shape", [(2, 4, 3), (5, 1, 30), (3, 16, 28), (4, 17, 29), (9, 21, 57), (70, 33, 31),
+                                   (6, 420, 421), (8, 362, 364)])
+@pytest.mark.parametrize("method", [0, 1])
+def test_sb_two_voxel_kernel_matches_the_one_voxel_kernel(method, shape, monkeypatch):
+    """Split-Bregman volumes on the two-voxel kernel: tile edges of both heights,
+    chunk edges, odd rows, arrays off 8-byte alignment, with and without the rule."""
+    import torch
+    from ccpi.filters import regularisersCuPy as R
+
+    rng = np.random.default_rng(7)
+    v = (rng.random(shape) * 0.2 + np.arange(shape[-1]) // 5 % 2).astype(np.float32)
+    for shift in (0, 1):
+        x = torch.empty(v.size + 1, dtype=torch.float32, device="cuda")[shift:shift + v.size].view(shape)
+        x.copy_(torch.from_numpy(v))
+        for tol in (0.0, 1e-7):
+            got = R.SB_TV(x, 0.05, 15, tol, method).cpu().numpy()
+            monkeypatch.setenv("CILREG_SB_KERNEL", "tiled")
+            want = R.SB_TV(x, 0.05, 15, tol, method).cpu().numpy()
+            monkeypatch.delenv("CILREG_SB_KERNEL")
+            np.testing.assert_allclose(got, want, rtol=0, atol=1e-5 * float(np.ptp(want)))
