@@ -5,6 +5,8 @@
 // those kernels.
 #pragma once
 
+#include <float.h>
+
 #include <type_traits>
 
 #include "runtime.cuh"
@@ -45,6 +47,17 @@ __device__ __forceinline__ float2 rcp2(float2 x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
     return fma2(r, fma2(neg2(x), r, make_float2(1.0f, 1.0f)), r);
+}
+
+// sqrt(sq) and its reciprocal per component from one approximate reciprocal
+// square root: sqrt(sq) by Heron's step on sq rsqrt(sq), the reciprocal by
+// Newton's step, each within an ulp and issued paired.  FLT_MIN keeps sq = 0
+// finite (norm 0).
+__device__ __forceinline__ void norm2(float2 sq, float2& norm, float2& inverse) {
+    const float2 rs = make_float2(rsqrtf(fmaxf(sq.x, FLT_MIN)), rsqrtf(fmaxf(sq.y, FLT_MIN)));
+    norm = mul2(sq, rs);
+    norm = fma2(mul2(splat(0.5f), rs), fma2(neg2(norm), norm, sq), norm);
+    inverse = fma2(rs, fma2(neg2(norm), rs, splat(1.0f)), rs);
 }
 
 // Rows of odd length (3D): the last pair's second voxel lies beyond the row and

@@ -28,7 +28,6 @@
 //   C.  publishes U^k of plane j (loaded one step earlier).
 // One barrier per plane.  Odd rows (a last pair whose second voxel is the
 // mirrored one) and arrays off 8-byte alignment run the 4-byte instantiation.
-#include <float.h>
 #include <stdlib.h>
 
 #include "pair.cuh"
@@ -58,12 +57,8 @@ __device__ __forceinline__ void shrink(const float2 (&g)[3], const float2 (&b)[3
         for (int c = 0; c < 3; c++) dd[c] = make_float2(one(v[c].x), one(v[c].y));
     } else {
         const float2 sq = fma2(v[2], v[2], fma2(v[0], v[0], mul2(v[1], v[1])));
-        // |v| by Heron's step on sq rsqrt(sq), 1/|v| by Newton's step on
-        // rsqrt(sq): each within an ulp.  FLT_MIN keeps v = 0 finite (D = 0).
-        const float2 rs = make_float2(rsqrtf(fmaxf(sq.x, FLT_MIN)), rsqrtf(fmaxf(sq.y, FLT_MIN)));
-        float2 den = mul2(sq, rs);
-        den = fma2(mul2(splat(0.5f), rs), fma2(neg2(den), den, sq), den);
-        const float2 r = fma2(rs, fma2(neg2(den), rs, splat(1.0f)), rs);
+        float2 den, r;
+        norm2(sq, den, r);
         const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
 #pragma unroll
         for (int c = 0; c < 3; c++) dd[c] = mul2(m, mul2(v[c], r));
@@ -98,7 +93,7 @@ __global__ void __launch_bounds__(LX * ROWS, 2) k_sb_pair(SbFusedArgs a, Dims d,
     const int o = (ty * LX + tx) * 2, oyl = (yl * LX + tx) * 2, oyh = (yh * LX + tx) * 2;
     const int col = min(max(y, 0), ny - 1) * nx + (ALIGNED ? min(max(X, 0), nx - 2) : pair_col(X, nx));
     const int dc = ALIGNED ? 1 : pair_step(X, nx);
-    const float2 lam2 = splat(a.lambda), mu2 = splat(a.mu), norm2 = splat(a.norm);
+    const float2 lam2 = splat(a.lambda), mu2 = splat(a.mu), nrm2 = splat(a.norm);
     const float dlam = a.dlam;
     float2 pa = splat(0.f), pb = splat(0.f);
     const int z0 = blockIdx.z * zc;
@@ -183,7 +178,7 @@ __global__ void __launch_bounds__(LX * ROWS, 2) k_sb_pair(SbFusedArgs a, Dims d,
         float2 q = add2(above(ppu), below(ppu));
         q = add2(add2(q, ld2(sU[SM2] + oyh)), ld2(sU[SM2] + oyl));
         q = add2(add2(q, zh0), zl0);
-        const float2 u1 = mul2(norm2, fma2(add2(g, q), lam2, fb));
+        const float2 u1 = mul2(nrm2, fma2(add2(g, q), lam2, fb));
         st2(sU1[W2] + o, u1);
         // B. U2 of plane kf = j-3
         if (FULL) {
@@ -195,7 +190,7 @@ __global__ void __launch_bounds__(LX * ROWS, 2) k_sb_pair(SbFusedArgs a, Dims d,
             float2 p = add2(xh, xl);
             p = add2(add2(p, ld2(sU1[W3] + oyh)), ld2(sU1[W3] + oyl));
             p = add2(add2(p, zh1), zl1);
-            const float2 u2 = mul2(norm2, fma2(add2(gc, p), lam2, fc));
+            const float2 u2 = mul2(nrm2, fma2(add2(gc, p), lam2, fc));
             if (upd) {
                 put(a.u2 + (kf * sxy + col), u2);
                 if (CHECK) {

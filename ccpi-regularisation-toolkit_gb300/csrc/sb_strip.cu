@@ -24,25 +24,27 @@ struct Args {
     bool aniso;
 };
 
-// D = shrink(g + b) and B = b + (g - D) of a pair
-__device__ __forceinline__ void shrink(float2 g1, float2 g2, float2 b1, float2 b2, float dlam, bool aniso, float2& d1,
-                                       float2& d2, float2& n1, float2& n2) {
+// D = shrink(g + b) and B = b + (g - D) of a pair, as D - B and B
+__device__ __forceinline__ void shrink(float2 g1, float2 g2, float2 b1, float2 b2, float dlam, bool aniso, float2& q1,
+                                       float2& q2, float2& n1, float2& n2) {
     const float2 v1 = add2(g1, b1), v2 = add2(g2, b2);
+    float2 d1, d2;
     if (aniso) {
         // (v / |v|) * max(|v| - 1/lambda, 0), 0 for v == 0: the same value as a sign copy
         auto one = [&](float v) { return copysignf(fmaxf(fabsf(v) - dlam, 0.f), v); };
         d1 = make_float2(one(v1.x), one(v1.y));
         d2 = make_float2(one(v2.x), one(v2.y));
     } else {
-        const float2 sq = fma2(v1, v1, mul2(v2, v2));
-        const float2 den = make_float2(__fsqrt_rn(sq.x), __fsqrt_rn(sq.y));
+        float2 den, r;
+        pair::norm2(fma2(v1, v1, mul2(v2, v2)), den, r);
         const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
-        const float2 r = make_float2(den.x != 0.f ? __frcp_rn(den.x) : 0.f, den.y != 0.f ? __frcp_rn(den.y) : 0.f);
         d1 = mul2(m, mul2(v1, r));
         d2 = mul2(m, mul2(v2, r));
     }
     n1 = add2(b1, sub2(g1, d1));
     n2 = add2(b2, sub2(g2, d2));
+    q1 = sub2(d1, n1);
+    q2 = sub2(d2, n2);
 }
 
 template <int R, bool CHECK>
@@ -55,23 +57,22 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
     for (int r = 0; r < R; r++) muf[r] = mul2(splat(a.mu), q.load_const(a.f, r));  // before the wait
     if (!begin<CHECK>(fr)) return;
     const bool top = q.Y == 0;
-    float2 d1[R], d2[R], d2up = splat(0.f), b2up = splat(0.f);
+    float2 q1[R], q2[R], q2up = splat(0.f);  // D - B
 #pragma unroll
     for (int r = 0; r < R; r++) {
         u[r] = q.load(a.u, r);
         b1[r] = a.bp[0] ? q.load(a.bp[0], r) : splat(0.f);
         b2[r] = a.bp[0] ? q.load(a.bp[1], r) : splat(0.f);
-        d1[r] = d2[r] = splat(0.f);
+        q1[r] = q2[r] = splat(0.f);
     }
     if (a.first && a.d0[0]) {  // given D^0, B^0: of the rows and of the one above
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            d1[r] = q.load(a.d0[0], r);
-            d2[r] = q.load(a.d0[1], r);
+            q1[r] = sub2(q.load(a.d0[0], r), b1[r]);
+            q2[r] = sub2(q.load(a.d0[1], r), b2[r]);
         }
         const int up = top ? 1 : -1;  // row -1 of the image is the mirrored row 1
-        d2up = q.load(a.d0[1], up);
-        b2up = q.load(a.bp[1], up);
+        q2up = sub2(q.load(a.d0[1], up), q.load(a.bp[1], up));
     }
     const float2 lam2 = splat(a.lambda), norm2 = splat(a.norm);
     float2 pa = splat(0.f), pb = splat(0.f);
@@ -81,13 +82,13 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
     // D, B, their divergence term G and the first sweep
     auto sweep1 = [&](auto edge_, float2 above, float2 next, float2 below, float2 b1a, float2 b2a, bool given) {
         constexpr bool EDGE = decltype(edge_)::value;
-        if (!given) {  // the row above: D2 and B2
-            float2 c = above, e1, n1;
+        if (!given) {  // the row above: its y component
+            float2 c = above, e1, n1, n2;
             float lo, hi;
             x_neighbours<EDGE>(q, c, lo, hi);
-            shrink(sub2(make_float2(c.y, hi), c), sub2(next, c), b1a, b2a, a.dlam, a.aniso, e1, d2up, n1, b2up);
+            shrink(sub2(make_float2(c.y, hi), c), sub2(next, c), b1a, b2a, a.dlam, a.aniso, e1, q2up, n1, n2);
         }
-        float2 um = above, dl = d2up, bl = b2up;
+        float2 um = above, ql = q2up;
 #pragma unroll
         for (int r = 0; r < R; r++) {
             float2 c = u[r];
@@ -98,25 +99,19 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
             if (EDGE && r == q.bottom) uh = um;
             if (!given) {
                 float2 n1, n2;
-                shrink(sub2(xh, c), sub2(uh, c), b1[r], b2[r], a.dlam, a.aniso, d1[r], d2[r], n1, n2);
+                shrink(sub2(xh, c), sub2(uh, c), b1[r], b2[r], a.dlam, a.aniso, q1[r], q2[r], n1, n2);
                 b1[r] = n1;
                 b2[r] = n2;
             }
-            float dxl = left_of(d1[r]), bxl = left_of(b1[r]);
-            if (EDGE && q.at_left) {
-                dxl = d1[r].y;
-                bxl = b1[r].y;
-            }
+            float qxl = left_of(q1[r]);
+            if (EDGE && q.at_left) qxl = q1[r].y;
             // Dx[-1] - Dx + Dy[-1] - Dy - Bx[-1] + Bx - By[-1] + By (SB_TV_core.c:166)
-            float2 s = sub2(make_float2(dxl, d1[r].x), d1[r]);
-            s = sub2(add2(s, dl), d2[r]);
-            s = add2(sub2(s, make_float2(bxl, b1[r].x)), b1[r]);
-            s = add2(sub2(s, bl), b2[r]);
+            float2 s = sub2(make_float2(qxl, q1[r].x), q1[r]);
+            s = sub2(add2(s, ql), q2[r]);
             g[r] = s;
             u1[r] = mul2(norm2, fma2(add2(s, sum4(xh, xl, uh, um)), lam2, muf[r]));
             um = u[r];
-            dl = d2[r];
-            bl = b2[r];
+            ql = q2[r];
         }
     };
     auto sweep2 = [&](auto edge_, float2 above, float2 below, bool sum) {
@@ -189,7 +184,7 @@ bool sb_strip_applies(const Dims& d) {
 
 int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, int iters, float epsil, const Dims& d,
                  cudaStream_t s, float* info, SbWarm* warm) {
-    static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 1620.0, 685.0, 1000.0, 800.0};
+    static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 910.0, 430.0, 870.0, 1070.0};
     const bool checking = epsil != 0.0f;
     const Plan P = plan(d.nx, d.ny, iters, checking, choices);
     Scratch scratch(s);
