@@ -49,6 +49,15 @@ __device__ __forceinline__ float2 rcp2(float2 x) {
     return fma2(r, fma2(neg2(x), r, make_float2(1.0f, 1.0f)), r);
 }
 
+// a * b per component, never merged with a following addition.  A paired
+// product whose only use is a paired addition becomes a fused multiply-add
+// (measured: ROF's last row of a strip differed in the last place from the
+// one-iteration kernel, whose products go through shared memory); two scalar
+// products do not.
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
+    return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+
 // sqrt(sq) and its reciprocal per component from one approximate reciprocal
 // square root: sqrt(sq) by Heron's step on sq rsqrt(sq), the reciprocal by
 // Newton's step, each within an ulp and issued paired.  FLT_MIN keeps sq = 0

@@ -122,7 +122,11 @@ int pd_run(const float* f, float* u_out, float lam, int iters, float epsil, floa
     // CILREG_PD_KERNEL=simple selects the per-voxel kernel (kept for A/B checks)
     const char* ek = getenv("CILREG_PD_KERNEL");
     const bool stream = !(ek && strcmp(ek, "simple") == 0);
-    const PdPlan T = pd_stream_plan(d);
+    const PdPlan P = pd_pair_plan(d, ((uintptr_t)f | (uintptr_t)u_out) % 8 == 0);
+    const PdPlan T = P.pair ? P : pd_stream_plan(d);
+    auto step = [&](const PdStreamArgs& b, const StopCtl* c, double2* parts, cudaStream_t st) {
+        return T.pair ? pd_pair_step(T, b, d, c, parts, st) : pd_stream_step(T, b, d, c, parts, st);
+    };
     const long long nparts = stream ? T.nblocks : num_blocks(L);
     IterControl ctl(s, scratch, iters, epsil, nparts);
     CILREG_TRY(ctl.status());
@@ -161,7 +165,7 @@ int pd_run(const float* f, float* u_out, float lam, int iters, float epsil, floa
             b.nonneg = (nonneg == 1);
             b.aniso = (methodTV != 0);
             b.check = 0;
-            CILREG_TRY(pd_stream_step(T, b, d, ctl.ctl(), ctl.partials(), st));
+            CILREG_TRY(step(b, ctl.ctl(), ctl.partials(), st));
             note_launch();
             return OK;
         }));
@@ -204,7 +208,7 @@ int pd_run(const float* f, float* u_out, float lam, int iters, float epsil, floa
             b.nonneg = a.nonneg;
             b.aniso = a.aniso;
             b.check = check;
-            CILREG_TRY(pd_stream_step(T, b, d, ctl.ctl(), ctl.partials(), s));
+            CILREG_TRY(step(b, ctl.ctl(), ctl.partials(), s));
         } else if (three) {
             k_pd_step<true><<<L.grid, L.block, 0, s>>>(a, d, L.kz, ctl.ctl(), ctl.partials());
         } else {

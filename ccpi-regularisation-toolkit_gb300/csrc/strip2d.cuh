@@ -230,15 +230,6 @@ struct Place {
     }
 };
 
-// a * b per component, never merged with a following addition.  A paired
-// product whose only use is a paired addition becomes a fused multiply-add
-// (measured: ROF's last row of a strip differed in the last place from the
-// one-iteration kernel, whose products go through shared memory); two scalar
-// products do not.
-__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
-    return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-}
-
 // 1/sqrt(s) for normal s: the flush-to-zero form of rsqrtf's approximation,
 // the same value without the scaling that subnormal arguments need
 __device__ __forceinline__ float rsqrt_normal(float s) {
