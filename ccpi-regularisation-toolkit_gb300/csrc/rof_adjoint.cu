@@ -213,12 +213,15 @@ int rof_vjp_run(const float* f, const float* ybar, float lam, int iters, float t
     CILREG_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), s));
     CILREG_CUDA(cudaMemsetAsync(fbar, 0, nb, s));
 
+    // The states run odd rows one voxel per thread: the two-voxel kernel rounds
+    // some sums otherwise, and the reverse sweep, discontinuous in the states,
+    // turns their last places into 1e-6 of the 64-bit lambda derivative.
     // pass 1: forward from f up to the last segment start, keeping U there
     // and at every earlier segment start
     const float* cur = f;
     for (int k = 0; k < (nseg - 1) * ckpt; k++) {
         float* nxt = ((k + 1) % ckpt == 0) ? ck[(k + 1) / ckpt] : ping[k & 1];
-        CILREG_TRY(rof_launch_step(cur, nxt, f, nullptr, lam, tau, d, ctl, 0, nullptr, s));
+        CILREG_TRY(rof_launch_step(cur, nxt, f, nullptr, lam, tau, d, ctl, 0, nullptr, s, false));
         cur = nxt;
     }
 
@@ -230,7 +233,7 @@ int rof_vjp_run(const float* f, const float* ybar, float lam, int iters, float t
         const float* start = (g == 0) ? f : ck[g];
         auto state = [&](int k) -> const float* { return (k == k0) ? start : seg[k - k0]; };
         for (int k = k0; k + 1 < k1; k++)
-            CILREG_TRY(rof_launch_step(state(k), seg[k + 1 - k0], f, nullptr, lam, tau, d, ctl, 0, nullptr, s));
+            CILREG_TRY(rof_launch_step(state(k), seg[k + 1 - k0], f, nullptr, lam, tau, d, ctl, 0, nullptr, s, false));
         for (int k = k1 - 1; k >= k0; k--) {
             RofAdjArgs a;
             a.u = state(k);

@@ -12,11 +12,12 @@ struct RofPlan {
     bool pair = false;  // the two-voxels-per-thread kernel (rof_pair.cu)
 };
 
-RofPlan rof_tiled_plan(const Dims& d);
+// odd_pairs: volumes with odd rows run the two-voxel kernel too
+RofPlan rof_tiled_plan(const Dims& d, bool odd_pairs = true);
 
-// volumes and images with nx even and fewer than 2^31 voxels run k_rof_pair
-// (3D) or k_rof_pair2d (CILREG_ROF_KERNEL=async, reg or simple select a
-// one-voxel kernel)
+// volumes of fewer than 2^31 voxels run k_rof_pair; of 2D images those with nx
+// even that do not run strips run k_rof_pair2d (CILREG_ROF_KERNEL=async, reg or
+// simple select a one-voxel kernel)
 bool rof_pair_applies(const Dims& d);
 RofPlan rof_pair_plan(const Dims& d);
 int rof_pair_step(const RofPlan& T, const float* cur, float* nxt, const float* f, const float* lam_arr, float lam,

@@ -322,3 +322,26 @@ def test_fgp_vjp_of_a_batch_equals_single_calls(shape, iters):
         np.testing.assert_array_equal(fbar[v].cpu().numpy(), one.cpu().numpy())
         # the same FP32 sums per column of planes, added in FP64 in another order
         np.testing.assert_allclose(lbar[v], l1[0], rtol=1e-9, atol=1e-9)
+
+
+def test_rof_adjoint_states_of_odd_rows_run_one_voxel_per_thread(monkeypatch):
+    """Volumes with odd rows: the same gradients as with the one-voxel kernel
+    throughout (the 64-bit lambda derivative follows the states' last places)."""
+    import torch
+    from ccpi.filters import autograd as A
+
+    rng = np.random.default_rng(11)
+    for shape in ((26, 40, 103), (5, 17, 31)):
+        f0 = torch.from_numpy((rng.random(shape) * 0.1 + np.arange(shape[-1]) // 9 % 2).astype(np.float32)).cuda()
+        ybar = torch.from_numpy(rng.standard_normal(shape).astype(np.float32)).cuda()
+        got = []
+        for kernel in ("", "async"):
+            if kernel:
+                monkeypatch.setenv("CILREG_ROF_KERNEL", kernel)
+            f = f0.clone().requires_grad_()
+            lam = torch.tensor(0.02, dtype=torch.float64, requires_grad=True)
+            A.rof_tv(f, lam, 38, 0.001, checkpoint=10).backward(ybar)
+            got.append((f.grad.cpu().numpy(), float(lam.grad)))
+        monkeypatch.delenv("CILREG_ROF_KERNEL")
+        np.testing.assert_array_equal(got[0][0], got[1][0])
+        assert got[0][1] == got[1][1]
