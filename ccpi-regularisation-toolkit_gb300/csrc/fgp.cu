@@ -141,9 +141,12 @@ int fgp_run(const float* f, float* u_out, float lam, int iters, float epsil, int
     if (tma) {
         T = fgp_tiled_plan(d, fgp_tma_resident());
     } else if (T.use && !TP.use) {
-        // below the tensor-copy kernel's sizes: two voxels per thread
+        // below the tensor-copy kernel's sizes: two voxels per thread, even rows
+        // from 2^21 voxels in k_fgp_x2, smaller and odd ones by shuffles
         const TiledPlan X = fgp_x2_plan(d);
+        const TiledPlan Y = X.use ? TiledPlan{} : fgp_shfl_plan(d);
         if (X.use) T = X;
+        if (Y.use) T = Y;
     }
     IterControl ctl(s, scratch, iters, epsil, T.use ? T.nblocks : num_blocks(L));
     CILREG_TRY(ctl.status());

@@ -492,6 +492,9 @@ int fgp_tiled_step(const TiledPlan& T, const float* const pc[3], const float* co
     if (T.x2 && (!b || d.nz == 1))
         return fgp_x2_step(T, pc, po, pn, f, u, lam, c, multip, nonneg, aniso, write_u, write_p, check, d, ctl,
                            partials, s, carr, cbase, coff, b);
+    if (T.shfl && !b)
+        return fgp_shfl_step(T, pc, po, pn, f, u, lam, c, multip, nonneg, aniso, write_u, write_p, check, d, ctl,
+                             partials, s, carr, cbase, coff);
     TiledArgs a;
     a.carr = carr;
     a.cbase = cbase;

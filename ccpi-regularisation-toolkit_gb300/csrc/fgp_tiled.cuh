@@ -13,7 +13,8 @@ struct TiledPlan {
     dim3 grid, block;
     long long nblocks = 0;
     int zchunk = 0;
-    bool x2 = false;  // the two-voxels-per-thread kernel (fgp_x2.cu)
+    bool x2 = false;    // the two-voxels-per-thread kernel (fgp_x2.cu)
+    bool shfl = false;  // the same with neighbours by shuffles (fgp_shfl.cu)
 };
 
 // z chunks balanced for `resident_ctas_per_sm` CTAs per SM (0: those of k_fgp_stream)
@@ -42,6 +43,15 @@ int fgp_x2_step(const TiledPlan& T, const float* const pc[3], const float* const
                 const float* f, float* u, float lam, float c, float multip, int nonneg, int aniso, int write_u,
                 int write_p, int check, const Dims& d, const StopCtl* ctl, double2* partials, cudaStream_t s,
                 const float* carr, const int* cbase, int coff, const float* const* b = nullptr);
+
+// The iteration with two voxels per thread and x neighbours by shuffles
+// (fgp_shfl.cu): 3D volumes below 2^23 voxels, rows of any length from two,
+// k_fgp_stream's bits (CILREG_FGP_KERNEL=stream or simple keep that kernel)
+TiledPlan fgp_shfl_plan(const Dims& d);
+int fgp_shfl_step(const TiledPlan& T, const float* const pc[3], const float* const po[3], float* const pn[3],
+                  const float* f, float* u, float lam, float c, float multip, int nonneg, int aniso, int write_u,
+                  int write_p, int check, const Dims& d, const StopCtl* ctl, double2* partials, cudaStream_t s,
+                  const float* carr, const int* cbase, int coff);
 
 // Two iterations k, k+1 in one streaming pass (fgp_pair.cu; 3D only).
 struct PairPlan {

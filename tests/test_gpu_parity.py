@@ -794,3 +794,24 @@ def test_pd_two_voxel_kernel_matches_the_one_voxel_kernel(method, shape, monkeyp
             want = R.PD_TV(x, 0.05, 15, tol, method, nonneg).cpu().numpy()
             monkeypatch.delenv("CILREG_PD_KERNEL")
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("shape", [(2, 4, 3), (5, 1, 30), (3, 14, 28), (4, 15, 29), (9, 29, 57), (70, 33, 32)])
+@pytest.mark.parametrize("method", [0, 1])
+def test_fgp_shuffle_kernel_matches_the_one_voxel_kernel(method, shape, monkeypatch):
+    """Small FGP-TV volumes with x neighbours by shuffles: tile and chunk edges,
+    odd rows, arrays off 8-byte alignment, with and without the rule; the same bits."""
+    import torch
+    from ccpi.filters import regularisersCuPy as R
+
+    rng = np.random.default_rng(9)
+    v = (rng.random(shape) * 0.4 - 0.1 + np.arange(shape[-1]) // 5 % 2).astype(np.float32)
+    for shift in (0, 1):
+        x = torch.empty(v.size + 1, dtype=torch.float32, device="cuda")[shift:shift + v.size].view(shape)
+        x.copy_(torch.from_numpy(v))
+        for tol, nonneg in ((0.0, 0), (1e-7, 1)):
+            got = R.FGP_TV(x, 0.05, 70, tol, method, nonneg).cpu().numpy()
+            monkeypatch.setenv("CILREG_FGP_KERNEL", "stream")
+            want = R.FGP_TV(x, 0.05, 70, tol, method, nonneg).cpu().numpy()
+            monkeypatch.delenv("CILREG_FGP_KERNEL")
+            np.testing.assert_array_equal(got, want)
