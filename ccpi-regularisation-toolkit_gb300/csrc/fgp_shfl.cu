@@ -185,7 +185,63 @@ __global__ void __launch_bounds__(NTF, 4) k_fgp_shfl(ShflArgs a, Dims d, int zc,
     if (CHECK) block_pair_partial<NTF>(pa, pb, partials, block_slot());
 }
 
+// one iteration of every volume of a batch of one shape, a flat grid over all
+// tiles (the states of the adjoint)
+__global__ void __launch_bounds__(NTF, 4) k_fgp_shfl_batch(const FgpBatchVol* __restrict__ vols,
+                                                           const int* __restrict__ tile_vol, int it, float c,
+                                                           int nonneg, int aniso) {
+    pdl_wait();  // the previous iteration has completed (launch_pdl)
+    if (pdl_many_waves()) pdl_trigger();
+    const FgpBatchVol& V = vols[tile_vol[blockIdx.x]];
+    // the volume's pointers and extents in shared memory: in registers they spill
+    __shared__ ShflArgs a;
+    __shared__ Dims d;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int q = 0; q < 3; q++) {
+            a.pn[q] = V.ring[it % 3][q];
+            a.pc[q] = V.ring[(it + 2) % 3][q];
+            a.po[q] = V.ring[(it + 1) % 3][q];
+        }
+        a.f = V.f;
+        a.u = V.u;
+        a.lam = V.lam;
+        a.multip = V.multip;
+        a.nonneg = nonneg;
+        a.aniso = aniso;
+        a.write_u = 0;
+        a.write_p = 1;
+        d = V.d;
+    }
+    __syncthreads();
+    const int lt = (int)(blockIdx.x - V.tile_base), gx = V.gx, gy = V.gy;
+    const int bx = lt % gx, by = (lt / gx) % gy, bz = lt / (gx * gy);
+    float pa, pb;
+    if (V.aligned)
+        shfl_tile<false, true>(a, d, V.zc, bx, by, bz, c, pa, pb);
+    else
+        shfl_tile<false, false>(a, d, V.zc, bx, by, bz, c, pa, pb);
+    if (!pdl_many_waves()) pdl_trigger();
+}
+
 }  // namespace
+
+bool fgp_shfl_tile_grid(const Dims& d, int nvol, int& gx, int& gy, int& gz, int& zc) {
+    if (!(d.nz > 1 && pair_rows(d))) return false;
+    static const int resident = resident_ctas(k_fgp_shfl_batch, NTF);
+    gx = (d.nx + OXF - 1) / OXF;
+    gy = (d.ny + OYF - 1) / OYF;
+    zc = wave_zchunk((long long)gx * gy * nvol, d.nz, resident, 2, ZCHUNK, 2.5);
+    gz = (d.nz + zc - 1) / zc;
+    return true;
+}
+
+int fgp_shfl_batch_step(const FgpBatchVol* d_vols, const int* d_tile_vol, long long ntiles, int it, float c,
+                        int nonneg, int aniso, cudaStream_t s) {
+    if (ntiles < 1 || ntiles > 2147483647LL) return fail(ERR_ARG, __FILE__, __LINE__, "tile count %lld", ntiles);
+    CILREG_CUDA(launch_pdl(k_fgp_shfl_batch, dim3((unsigned)ntiles), dim3(LX, ROWS, 1), 0, s, d_vols, d_tile_vol, it, c,
+                           nonneg, aniso));
+    return OK;
+}
 
 TiledPlan fgp_shfl_plan(const Dims& d) {
     TiledPlan T;

@@ -97,6 +97,7 @@ struct FgpBatchVol {
     float lam, multip;
     long long tile_base; // first flat tile index of this volume
     int gx, gy, gz, zc;  // tile grid and z chunk of this volume
+    int aligned;         // of fgp_shfl_batch_step: nx even, every array 8-byte aligned
 };
 
 // Persistent batched run (one launch for every iteration of every volume):
@@ -137,6 +138,13 @@ bool fgp_x2_batch_usable(const Dims* dims, const float* const* f, float* const* 
 void fgp_x2_tile_grid(const Dims& d, int zc, int& gx, int& gy, int& gz);
 int fgp_x2_batch_step(const FgpBatchVol* d_vols, const int* d_tile_vol, long long ntiles, int it, float c,
                       int nonneg, int aniso, int write_u, int write_p, int check, cudaStream_t s);
+
+// an iteration of `nvol` volumes of one shape with the tile of fgp_shfl.cu,
+// without U, a rule or stopped volumes (the adjoint's states); its tile grid and
+// z chunk, false where the tile does not serve the shape
+bool fgp_shfl_tile_grid(const Dims& d, int nvol, int& gx, int& gy, int& gz, int& zc);
+int fgp_shfl_batch_step(const FgpBatchVol* d_vols, const int* d_tile_vol, long long ntiles, int it, float c,
+                        int nonneg, int aniso, cudaStream_t s);
 
 // 2D images run several iterations per launch (fgp_strip.cu; CILREG_FGP_KERNEL
 // or CILREG_STRIP2D=0 keep one per launch).  cseq: the momentum coefficient of
