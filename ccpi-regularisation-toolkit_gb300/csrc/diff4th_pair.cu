@@ -27,8 +27,8 @@
 // W on the inner 30 x (ROWS-2) points, the update on the inner 28 x (ROWS-4),
 // whole pairs (threads 1..14 of rows 2..ROWS-3).  Tile x origins are even
 // (x0 = 28 bx - 2).  Odd rows (a last pair whose second voxel is the mirrored
-// one: 1150 -> 788 us per 511^3 iteration against k_d4_stream) and arrays off 8-byte alignment run the
-// 4-byte instantiation.
+// one: 1150 -> 788 us per 511^3 iteration against k_d4_stream) and arrays off
+// 8-byte alignment run the 4-byte instantiation.
 #include <stdlib.h>
 
 #include "diff4th_tiled.cuh"

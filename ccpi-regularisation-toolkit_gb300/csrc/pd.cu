@@ -1,6 +1,9 @@
 // PD-TV: Chambolle-Pock primal-dual TV denoising (reference: PD_TV_core.c:40-252).
 //
-// One fused kernel per iteration.  State: the extrapolated primal iterate
+// One fused kernel per iteration: 3D volumes two voxels per thread
+// (pd_pair.cu), 2D images several iterations per launch (pd_strip.cu), others
+// k_pd_stream and k_pd_2d (pd_tiled.cu); k_pd_step below one voxel per thread
+// without a stream (CILREG_PD_KERNEL=simple).  State: the extrapolated primal iterate
 // Ue (the reference's U after getX) and the dual P, both ping-ponged; the
 // kernel recomputes the projected dual at the voxel and at its three lower
 // neighbours, so P never makes a second pass through HBM.  Traffic per

@@ -23,8 +23,8 @@
 // A CTA of 16 x 16 threads holds a 32 x 16 tile with a one-voxel halo; the
 // inner 30 x 14 voxels are updated.  Tile x origins are even (x0 = 30 bx - 2)
 // so that the pairs of a tile are the pairs of the volume; the 8-byte accesses
-// need nx even and 8-byte aligned arrays (ALIGNED; the
-// other instantiation issues two 4-byte accesses instead).
+// need nx even and 8-byte aligned arrays (ALIGNED; the other instantiation
+// issues two 4-byte accesses instead, and serves odd rows).
 #include <stdlib.h>
 
 #include <type_traits>
