@@ -237,8 +237,7 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
         for (int t = 0; t < sp.count; t++) a.c[t] = cseq[sp.first + t];
         a.u = (checking && ((nl - 1 - k) & 1)) ? ualt : u_out;
         a.write_u = end || sp.check;
-        CILREG_CUDA(launch_pdl(b ? pick<true>(P.R, checking) : pick<false>(P.R, checking), grid_of(P, fr, checking),
-                               dim3(32, NW, 1), 0, s, a, fr));
+        CILREG_CUDA(launch_strip(b ? pick<true>(P.R, checking) : pick<false>(P.R, checking), P, fr, checking, s, a));
         return OK;
     }));
     StopCtl done;

@@ -201,9 +201,9 @@ __global__ void __launch_bounds__(NTP, 4) k_fgp_x2(X2Args a, Dims d, int zc, con
 // on the inner 30 x 14 pixels; two barriers.  DTV: the FGP-dTV iteration,
 // R and the gradient of U each taken onto the complement of the reference's
 // unit gradient b at the pixel (FGP_dTV_core.c:311-314, 350-356).
-// Tile (bx, by) of one image; `wait` runs once f (and b) are loaded and
-// returns false when the run has stopped (the tile then does nothing and
-// returns false).
+// Tile (bx, by) of one image; `wait` runs before anything is loaded (a run's
+// first launch may follow the caller's kernel directly) and returns false when
+// the run has stopped (the tile then does nothing and returns false).
 template <bool CHECK, bool ALIGNED, bool DTV, class Wait>
 __device__ __forceinline__ bool x2_tile_2d(const X2Args& a, const Dims& d, int bx, int by, Wait wait, float& pa_out,
                                            float& pb_out) {
@@ -232,13 +232,13 @@ __device__ __forceinline__ bool x2_tile_2d(const X2Args& a, const Dims& d, int b
         if (ALIGNED) return __ldg(reinterpret_cast<const float2*>(p));
         return make_float2(__ldg(p), __ldg(p + 1));
     };
-    const float2 fv = in_xy ? ldg2(a.f + col) : splat(0.f);  // f never changes: loaded before the wait
-    float2 b1 = splat(0.f), b2 = splat(0.f);                  // neither does b
+    if (!wait()) return false;
+    const float2 fv = in_xy ? ldg2(a.f + col) : splat(0.f);
+    float2 b1 = splat(0.f), b2 = splat(0.f);
     if (DTV && in_xy) {
         b1 = ldg2(a.b[0] + col);
         b2 = ldg2(a.b[1] + col);
     }
-    if (!wait()) return false;
     float2 c1 = splat(0.f), o1 = splat(0.f), c2 = splat(0.f), o2 = splat(0.f);
     if (in_xy) {
         c1 = ldg2(a.pc[0] + col);

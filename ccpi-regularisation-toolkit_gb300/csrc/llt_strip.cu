@@ -159,8 +159,7 @@ int llt_strip_run(const float* f, float* u_out, float lam_rof, float lam_llt, in
     static const Choices choices = {2, 3, {2, 3, 4}, {2, 1, 1}, 1600.0, 850.0};
     return run_flow(choices, f, f, u_out, iters, epsil, d, s, info, true,
                     [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
-                        return launch_pdl(pick(P, rule), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam_rof,
-                                          lam_llt, tau, fr);
+                        return launch_strip(pick(P, rule), P, fr, rule, s, src, dst, f, lam_rof, lam_llt, tau);
                     });
 }
 

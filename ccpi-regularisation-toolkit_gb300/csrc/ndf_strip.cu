@@ -97,8 +97,7 @@ int ndf_strip_run(int pen, const float* f, float* u_out, float lam, float sg, fl
     static const Choices choices = {1, 3, {2, 4, 6}, {2, 2, 1}, 500.0, 250.0};
     return run_flow(choices, f, u_init ? u_init : f, u_out, iters, epsil, d, s, info, true,
                     [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
-                        return launch_pdl(pick(pen, P, rule), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam, sg,
-                                          isg, tau, fr);
+                        return launch_strip(pick(pen, P, rule), P, fr, rule, s, src, dst, f, lam, sg, isg, tau);
                     });
 }
 

@@ -192,8 +192,7 @@ int pd_strip_run(const float* f, float* u_out, float sigma, float tau, float lt,
                                  a.p[c] = k == 0 ? nullptr : pb[(k + 1) & 1][c];
                                  a.pn[c] = k == nl - 1 ? nullptr : pb[k & 1][c];
                              }
-                             CILREG_CUDA(launch_pdl(pick(P.R, checking), grid_of(P, fr, checking), dim3(32, NW, 1), 0,
-                                                    s, a, fr));
+                             CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
     StopCtl done;

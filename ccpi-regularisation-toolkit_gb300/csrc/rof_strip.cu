@@ -133,8 +133,7 @@ int rof_strip_run(const float* f, float* u_out, const float* lam_arr, float lam,
     const bool larr = lam_arr != nullptr;
     return run_flow(choices, f, u_init ? u_init : f, u_out, iters, epsil, d, s, info, !larr || host_aligned8(lam_arr),
                     [&](const Plan& P, bool rule, const Frame& fr, const float* src, float* dst) {
-                        return launch_pdl(pick(P, rule, larr), grid_of(P, fr, rule), dim3(32, NW, 1), 0, s, src, dst, f, lam_arr,
-                                          lam, tau, fr);
+                        return launch_strip(pick(P, rule, larr), P, fr, rule, s, src, dst, f, lam_arr, lam, tau);
                     });
 }
 

@@ -191,13 +191,24 @@ int run_replayed(int iters, int G, cudaStream_t s, Enq enqueue, Tail tail = Tail
 
 // Programmatic dependent launch: an iteration kernel launched with
 // launch_pdl may be scheduled while the kernel before it in the stream is
-// still draining; it runs pdl_wait() before its first memory access (the
-// previous grid has then completed and its writes are visible, so both the
-// read-after-write and the write-after-read order of ping-pong buffers hold)
-// and pdl_trigger() to let its own successor be scheduled early.  Both
-// instructions do nothing in a kernel launched without the attribute.
-// CILREG_PDL=0 launches normally (A/B checks).  launch_pdl returns the launch
-// status and clears it from the thread's error state.
+// still draining; it runs pdl_wait() before its first access to anything that
+// a kernel of the run writes (the previous grid has then completed and its
+// writes are visible, so both the read-after-write and the write-after-read
+// order of ping-pong buffers hold) and pdl_trigger() to let its own successor
+// be scheduled early.  Both instructions do nothing in a kernel launched
+// without the attribute.
+//
+// Some 2D kernels load the run's constant inputs (f, the lambda map, dTV's unit
+// gradient) before pdl_wait().  That is only in order when something of the run
+// already lies between the caller's last kernel and this launch: a caller's
+// kernel may have triggered its dependents while it still writes f, and even one
+// that never triggers is only sure to be seen after the wait.  So the first such
+// launch of a run either follows a copy or a memset of the run (which the stream
+// orders in full) or is launched without the attribute (launch_chained with
+// follows = false).
+//
+// CILREG_PDL=0 launches normally (A/B checks).  Both functions return the launch
+// status and clear it from the thread's error state.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 // Where a streaming kernel triggers.  At its start, the next grid's CTAs take
@@ -215,10 +226,11 @@ __device__ __forceinline__ bool pdl_many_waves() {
     return x * y * z >= 4096u;
 }
 bool pdl_enabled();
+// follows: the stream's last work is a kernel of the same run
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                       Args... args) {
-    if (!pdl_enabled()) {
+cudaError_t launch_chained(bool follows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                           Args... args) {
+    if (!follows || !pdl_enabled()) {
         kernel<<<grid, block, smem, s>>>(args...);
         return cudaGetLastError();
     }
@@ -235,6 +247,11 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ((KArgs)args)...);
     cudaGetLastError();  // the status is returned; leave no stale error behind
     return e;
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       Args... args) {
+    return launch_chained(true, kernel, grid, block, smem, s, args...);
 }
 
 // Deterministic reduction of a check's FP64 partials by one CTA of THREADS

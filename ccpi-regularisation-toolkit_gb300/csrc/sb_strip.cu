@@ -216,8 +216,7 @@ int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, in
                                  a.bp[c] = k > 0 ? bb[(k + 1) & 1][c] : warm ? warm->bb[c] : nullptr;
                                  a.bn[c] = (k == nl - 1 && !warm) ? nullptr : bb[k & 1][c];
                              }
-                             CILREG_CUDA(launch_pdl(pick(P.R, checking), grid_of(P, fr, checking), dim3(32, NW, 1), 0,
-                                                    s, a, fr));
+                             CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
     StopCtl done;

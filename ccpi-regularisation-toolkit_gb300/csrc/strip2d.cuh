@@ -128,6 +128,7 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
 struct Frame {
     int nx, ny, margin, count, gx;
     bool aligned;
+    bool follows;  // not the run's first launch
     const StopCtl* ctl;
     double2* partials;
     Finalize check;
@@ -148,8 +149,13 @@ __device__ __forceinline__ bool begin(const Frame& F) {
     }
     return !F.ctl->stop;
 }
-inline dim3 grid_of(const Plan& P, const Frame& F, bool rule) {
-    return rule ? dim3((unsigned)(P.nblocks + (F.check.n > 0 ? 1 : 0))) : dim3((unsigned)P.gx, (unsigned)P.gy);
+// Launches one launch of a run, `args` and then the frame.  The kernels load the
+// run's constant inputs before pdl_wait(), so the first launch, right behind
+// whatever wrote those inputs, waits for it in full like any kernel (launch_pdl).
+template <class Kernel, class... Args>
+cudaError_t launch_strip(Kernel kernel, const Plan& P, const Frame& F, bool rule, cudaStream_t s, Args... args) {
+    const dim3 grid = rule ? dim3((unsigned)(P.nblocks + (F.check.n > 0 ? 1 : 0))) : dim3((unsigned)P.gx, (unsigned)P.gy);
+    return launch_chained(F.follows, kernel, grid, dim3(32, NW, 1), 0, s, args..., F);
 }
 // one FP64 partial of the CTA's FP32 sums.  Two warps add the threads' sums
 // from shared memory: the FP64 unit takes 16 cycles for a warp's addition, and
@@ -304,7 +310,8 @@ int run_spans(const Plan& P, IterControl& ctl, int iters, bool checking, const D
     const int nl = count_spans(iters, P.T, checking);
     Finalize pending = {};
     return for_spans(iters, P.T, checking, [&](int k, const Span& sp) -> int {
-        const Frame fr{d.nx, d.ny, P.margin, sp.count, P.gx, aligned, ctl.ctl(), ctl.partials(k), pending};
+        const Frame fr{d.nx,  d.ny,      P.margin,        sp.count, P.gx,
+                       aligned, k > 0, ctl.ctl(), ctl.partials(k), pending};
         CILREG_TRY(each(k, sp, fr));
         note_launch();
         pending = Finalize{};

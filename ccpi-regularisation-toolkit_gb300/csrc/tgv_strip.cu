@@ -236,8 +236,7 @@ int tgv_strip_run(const float* f, float* u_out, float lam, float alpha1, float a
                                  a.s[c] = k == 0 ? nullptr : set[(k + 1) & 1][c];
                                  a.sn[c] = k == nl - 1 ? nullptr : set[k & 1][c];
                              }
-                             CILREG_CUDA(launch_pdl(pick(P.R, checking), grid_of(P, fr, checking), dim3(32, NW, 1), 0,
-                                                    s, a, fr));
+                             CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
     StopCtl done;
