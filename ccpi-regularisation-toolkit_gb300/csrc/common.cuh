@@ -20,11 +20,18 @@
 namespace cilreg {
 
 struct StopCtl {
-    int stop;     // 1 once the stopping rule has fired
+    int stop;     // 0 until the stopping rule has fired, then the number of the check that fired (at least 1)
     int iters;    // infovector[0]: the break index, or the requested count
     int count;    // cumulative number of checks with re < epsil
     float re;     // infovector[1]: the last relative change
 };
+
+// Whether a tile of a launch runs, given the stop flag it read.  `riding` is the
+// number of the check that one CTA of the same launch reduces meanwhile (0: none)
+// and that may set the flag to `riding` at any moment: only an earlier check's
+// stop holds for this launch, so the answer does not depend on that moment, and
+// every thread of a CTA gets the same one.
+__host__ __device__ inline bool tile_runs(int stop, int riding) { return stop == 0 || (riding > 0 && stop >= riding); }
 
 struct Dims {
     int nx, ny, nz;

@@ -129,7 +129,7 @@ struct Finalize {
     float epsil;
     int it;              // the check's iteration
     StopMirror* mirror;  // may be null
-    int seq;             // the check's number
+    int seq;             // the check's number, from 1; 0: not numbered
 };
 
 // Device-resident stopping control for one regulariser run.
@@ -282,10 +282,13 @@ __device__ __forceinline__ void finalize_check(const Finalize& f) {
             c.re = re;
             if (re < f.epsil) c.count += 1;
             if (c.count > 3) {
-                c.stop = 1;
+                c.stop = f.seq > 0 ? f.seq : 1;
                 c.iters = f.it;
             }
-            *f.ctl = c;
+            f.ctl->re = c.re;
+            f.ctl->count = c.count;
+            f.ctl->iters = c.iters;
+            *(volatile int*)&f.ctl->stop = c.stop;  // other CTAs of the launch may be reading it
             if (f.mirror) {
                 *(volatile int*)&f.mirror->ctl.stop = c.stop;
                 *(volatile int*)&f.mirror->ctl.iters = c.iters;

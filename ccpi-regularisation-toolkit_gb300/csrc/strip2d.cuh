@@ -119,8 +119,8 @@ inline Plan plan(int nx, int ny, int iters, bool checking, const Choices& c) {
 
 // What every launch gets besides its arrays: the image, the tiles, and the
 // check of the launch before, which CTA 0 then reduces while the others run.
-// The stop it may set holds from the launch after this one on, whose tiles
-// then leave both launches' results alone: launch k and k+1 write different
+// The stop it may set holds from the launch after this one on (tile_runs), whose
+// tiles then leave both launches' results alone: launch k and k+1 write different
 // buffers, so a run that stops at launch k's check ends on k's.  (A finalize
 // kernel between them cost 7 us per check.)  RULE: the run has a stopping rule;
 // the kernels of runs without one are compiled without all of this, which
@@ -147,7 +147,7 @@ __device__ __forceinline__ bool begin(const Frame& F) {
         finalize_check<NT>(F.check);
         return false;
     }
-    return !F.ctl->stop;
+    return tile_runs(*(const volatile int*)&F.ctl->stop, F.check.n > 0 ? F.check.seq : 0);
 }
 // Launches one launch of a run, `args` and then the frame.  The kernels load the
 // run's constant inputs before pdl_wait(), so the first launch, right behind
