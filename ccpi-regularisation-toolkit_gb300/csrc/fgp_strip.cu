@@ -240,19 +240,18 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
         CILREG_CUDA(launch_strip(b ? pick<true>(P.R, checking) : pick<false>(P.R, checking), P, fr, checking, s, a));
         return OK;
     }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
-        CILREG_CUDA(cudaMemcpyAsync(u_out, ualt, sizeof(float) * (size_t)d.n, cudaMemcpyDeviceToDevice, s));
-    if (warm && iters > 0) {
-        if (checking) {
-            const int k = done.stop ? span_of_check(done.iters) : nl - 1;
-            for (int c = 0; c < 2; c++)
-                CILREG_CUDA(cudaMemcpyAsync(warm->ring[to][c], set[k & 1][c], sizeof(float) * (size_t)d.n,
-                                            cudaMemcpyDeviceToDevice, s));
-        }
-        warm->base = (to + 1) % 3;
+    // what the check that fired, or the last launch, left: U, and a warm run's duals
+    SpanResult r[3];
+    int nr = 0;
+    if (checking && nl > 1) {
+        float* const ub[2] = {u_out, ualt};
+        r[nr++] = span_result(ub, nl, u_out);
     }
+    for (int c = 0; c < 2 && warm && checking && iters > 0; c++)
+        r[nr++] = SpanResult{{set[0][c], set[1][c]}, warm->ring[to][c], false};
+    if (nr > 0) CILREG_TRY(launch_take_span(ctl.ctl(), nl - 1, r, nr, d.n, s));
+    CILREG_TRY(ctl.finish(info));
+    if (warm && iters > 0) warm->base = (to + 1) % 3;
     return OK;
 }
 

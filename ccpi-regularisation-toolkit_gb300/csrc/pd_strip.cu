@@ -195,11 +195,11 @@ int pd_strip_run(const float* f, float* u_out, float sigma, float tau, float lt,
                              CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    if (done.stop)
-        CILREG_CUDA(cudaMemcpyAsync(u_out, brk[span_of_check(done.iters) & 1], bytes, cudaMemcpyDeviceToDevice, s));
-    return OK;
+    if (checking && iters > 0) {
+        const SpanResult r = {{brk[0], brk[1]}, u_out, true};
+        CILREG_TRY(launch_take_span(ctl.ctl(), nl - 1, &r, 1, d.n, s));
+    }
+    return ctl.finish(info);
 }
 
 }  // namespace cilreg

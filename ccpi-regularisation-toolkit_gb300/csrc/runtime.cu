@@ -383,6 +383,20 @@ __global__ void k_select_copy(const StopCtl* ctl, int iter_total, const float* b
     for (; i < n; i += stride) dst[i] = src[i];
 }
 
+struct SpanResults {
+    SpanResult r[3];
+};
+__global__ void k_take_span(const StopCtl* ctl, int last, SpanResults all, long long n) {
+    const SpanResult& r = all.r[blockIdx.y];
+    const int stop = ctl->stop;
+    if (!stop && r.stopped_only) return;
+    const float* src = r.src[(stop ? strip::span_of_check(ctl->iters) : last) & 1];
+    if (src == r.dst) return;
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (; i < n; i += stride) r.dst[i] = src[i];
+}
+
 static dim3 grid_stride_blocks(long long n) {
     long long b = (n + 255) / 256;
     if (b > 152LL * 16) b = 152LL * 16;
@@ -475,6 +489,18 @@ int launch_copy(float* dst, const float* src, long long n, cudaStream_t s) {
 int launch_select_pingpong(const StopCtl* ctl, int iter_total, float* const bufs[2], float* dst, long long n,
                            cudaStream_t s) {
     k_select_copy<<<grid_stride_blocks(n), 256, 0, s>>>(ctl, iter_total, bufs[0], bufs[1], dst, n);
+    note_launch();
+    CILREG_CUDA(cudaGetLastError());
+    return OK;
+}
+
+int launch_take_span(const StopCtl* ctl, int last, const SpanResult* results, int count, long long n, cudaStream_t s) {
+    if (count < 1 || count > 3) return fail(ERR_ARG, __FILE__, __LINE__, "%d results of a run", count);
+    SpanResults all = {};
+    for (int i = 0; i < count; i++) all.r[i] = results[i];
+    dim3 grid = grid_stride_blocks(n);
+    grid.y = count;
+    k_take_span<<<grid, 256, 0, s>>>(ctl, last, all, n);
     note_launch();
     CILREG_CUDA(cudaGetLastError());
     return OK;

@@ -325,6 +325,15 @@ int launch_copy(float* dst, const float* src, long long n, cudaStream_t s);
 // buffer bufs[(last+1) & 1] holds it (ping-pong with iteration it writing bufs[(it+1)&1]).
 int launch_select_pingpong(const StopCtl* ctl, int iter_total, float* const bufs[2], float* dst, long long n,
                            cudaStream_t s);
+// The same for runs of several iterations per launch (strip2d.cuh): launch k
+// wrote src[k & 1]; the result is that of the launch whose check fired, else of
+// launch `last` (nothing to copy where it lies in dst already).
+struct SpanResult {
+    const float* src[2];
+    float* dst;
+    bool stopped_only;  // dst is right already unless the rule fired
+};
+int launch_take_span(const StopCtl* ctl, int last, const SpanResult* results, int count, long long n, cudaStream_t s);
 
 
 template <class Enq, class Tail>

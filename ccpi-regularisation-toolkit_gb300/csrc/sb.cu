@@ -134,6 +134,27 @@ __global__ void __launch_bounds__(256) k_sb_shrink(SbArgs a, Dims d, int kz, con
 
 }  // namespace
 
+int sb_shrink2d(const SbSweepArgs& in, float dlam, bool aniso, const float* u, const SbWarm& warm, const Dims& d,
+                const StopCtl* ctl, cudaStream_t s) {
+    const Launch3 L = plan_launch(d);
+    SbArgs a = {};
+    for (int c = 0; c < 2; c++) {
+        a.dd[c] = warm.dd[c];
+        a.bb[c] = warm.bb[c];
+    }
+    a.u = u;
+    a.lambda = in.lambda;
+    a.mu = in.mu;
+    a.norm = in.norm;
+    a.dlam = dlam;
+    a.aniso = aniso;
+    a.f = in.f;
+    k_sb_shrink<false><<<L.grid, L.block, 0, s>>>(a, d, L.kz, ctl);
+    CILREG_CUDA(cudaGetLastError());
+    note_launch();
+    return OK;
+}
+
 int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int methodTV, const Dims& d,
            cudaStream_t s, float* info, SbWarm* warm) {
     CILREG_RANGE("cilreg SB-TV");
@@ -147,29 +168,7 @@ int sb_run(const float* f, float* u_out, float mu, int iters, float epsil, int m
         in.lambda = 2.0f * in.mu;
         in.norm = 1.0f / (in.mu + 4.0f * in.lambda);
         const float dlam = 1.0f / in.lambda;
-        CILREG_TRY(sb_strip_run(in, dlam, methodTV == 1, u_out, iters, epsil, d, s, info, warm));
-        if (warm && iters > 0) {  // D^n, B^n from the final U, in place
-            Scratch tmp(s);
-            StopCtl* never = (StopCtl*)tmp.bytes(sizeof(StopCtl));
-            if (!never) return tmp.status();
-            CILREG_CUDA(cudaMemsetAsync(never, 0, sizeof(StopCtl), s));
-            SbArgs a = {};
-            for (int c = 0; c < 2; c++) {
-                a.dd[c] = warm->dd[c];
-                a.bb[c] = warm->bb[c];
-            }
-            a.u = u_out;
-            a.lambda = in.lambda;
-            a.mu = in.mu;
-            a.norm = in.norm;
-            a.dlam = dlam;
-            a.aniso = (methodTV == 1);
-            a.f = f;
-            k_sb_shrink<false><<<L.grid, L.block, 0, s>>>(a, d, L.kz, never);
-            CILREG_CUDA(cudaGetLastError());
-            note_launch();
-        }
-        return OK;
+        return sb_strip_run(in, dlam, methodTV == 1, u_out, iters, epsil, d, s, info, warm);
     }
     Scratch scratch(s);
     const SbPlan T = sb_sweep2_plan(d);

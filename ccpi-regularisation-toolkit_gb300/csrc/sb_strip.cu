@@ -219,15 +219,20 @@ int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, in
                              CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    const int end = done.stop ? span_of_check(done.iters) : nl - 1;
-    if ((nl - 1 - end) & 1) CILREG_CUDA(cudaMemcpyAsync(u_out, ub[1], bytes, cudaMemcpyDeviceToDevice, s));
-    // a warm run leaves B of the iteration before its last U; the caller
-    // shrinks once more from that U
-    for (int c = 0; c < 2 && warm && iters > 0; c++)
-        CILREG_CUDA(cudaMemcpyAsync(warm->bb[c], bb[end & 1][c], bytes, cudaMemcpyDeviceToDevice, s));
-    return OK;
+    // what the check that fired, or the last launch, left: U, and a warm run's B of
+    // the iteration before, from which it shrinks once more with that U
+    SpanResult r[3];
+    int nr = 0;
+    if (checking && nl > 1) r[nr++] = span_result(ub, nl, u_out);
+    for (int c = 0; c < 2 && warm && iters > 0; c++) r[nr++] = SpanResult{{bb[0][c], bb[1][c]}, warm->bb[c], false};
+    if (nr > 0) CILREG_TRY(launch_take_span(ctl.ctl(), nl - 1, r, nr, d.n, s));
+    if (warm && iters > 0) {
+        StopCtl* never = (StopCtl*)scratch.bytes(sizeof(StopCtl));
+        if (!never) return scratch.status();
+        CILREG_CUDA(cudaMemsetAsync(never, 0, sizeof(StopCtl), s));
+        CILREG_TRY(sb_shrink2d(in, dlam, aniso, u_out, *warm, d, never, s));
+    }
+    return ctl.finish(info);
 }
 
 }  // namespace cilreg

@@ -54,10 +54,14 @@ int sb_pair_step(const SbPlan& T, const SbFusedArgs& a, bool aniso, const Dims& 
 
 // 2D images run several outer iterations per launch (sb_strip.cu;
 // CILREG_SB_KERNEL or CILREG_STRIP2D=0 keep one per launch).  `in` brings f and
-// the scalars; with `warm`, iteration 0 takes its D and B, and its bb receive
-// B^{n-1} of the n iterations run
+// the scalars; with `warm`, iteration 0 takes its D and B, which become those
+// after the n iterations run
 bool sb_strip_applies(const Dims& d);
 int sb_strip_run(const SbSweepArgs& in, float dlam, bool aniso, float* u_out, int iters, float epsil, const Dims& d,
                  cudaStream_t s, float* info, SbWarm* warm);
+
+// D^n and B^n of an image from its U^n and the B^{n-1} in warm.bb, in place (sb.cu)
+int sb_shrink2d(const SbSweepArgs& in, float dlam, bool aniso, const float* u, const SbWarm& warm, const Dims& d,
+                const StopCtl* ctl, cudaStream_t s);
 
 }  // namespace cilreg

@@ -274,7 +274,7 @@ inline int count_spans(int iters, int most, bool checking) {
     return checking ? 1 + (iters - 1 + 4) / 5 : (iters + most - 1) / most;
 }
 // index of the launch that runs check iteration `it`
-inline int span_of_check(int it) { return it / 5; }
+__host__ __device__ inline int span_of_check(int it) { return it / 5; }
 
 // the images that strips take
 inline bool applies(const Dims& d) { return d.nz == 1 && d.nx > 1 && d.ny > 1 && d.n < (1LL << 31) && enabled(); }
@@ -323,10 +323,17 @@ int run_spans(const Plan& P, IterControl& ctl, int iters, bool checking, const D
     });
 }
 
+// U of a run whose launch k writes bufs[(nl - 1 - k) & 1]
+inline SpanResult span_result(float* const bufs[2], int nl, float* dst) {
+    return SpanResult{{bufs[(nl - 1) & 1], bufs[nl & 1]}, dst, false};
+}
+
 // The run of a regulariser whose state is one image U beside f (ROF, NDF,
 // Diff4th, LLT-ROF): launch(plan, rule, frame, src, dst) enqueues one launch.
 // Launch k writes bufs[(nl - 1 - k) & 1], so the last writes u_out; a run that
-// stops early on the other buffer copies it.
+// stops early on the other buffer copies it.  The copy is chosen on the device
+// and enqueued before the call waits for the stream: the output is complete when
+// the call returns.
 template <class Launch>
 int run_flow(const Choices& choices, const float* f, const float* start, float* u_out, int iters, float epsil,
              const Dims& d, cudaStream_t s, float* info, bool aligned, Launch launch) {
@@ -346,11 +353,11 @@ int run_flow(const Choices& choices, const float* f, const float* start, float* 
         CILREG_CUDA(launch(P, checking, fr, k == 0 ? start : bufs[(nl - k) & 1], bufs[(nl - 1 - k) & 1]));
         return OK;
     }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
-        CILREG_CUDA(cudaMemcpyAsync(u_out, alt, bytes, cudaMemcpyDeviceToDevice, s));
-    return OK;
+    if (checking && nl > 1) {
+        const SpanResult r = span_result(bufs, nl, u_out);
+        CILREG_TRY(launch_take_span(ctl.ctl(), nl - 1, &r, 1, d.n, s));
+    }
+    return ctl.finish(info);
 }
 
 }  // namespace strip

@@ -239,11 +239,11 @@ int tgv_strip_run(const float* f, float* u_out, float lam, float alpha1, float a
                              CILREG_CUDA(launch_strip(pick(P.R, checking), P, fr, checking, s, a));
                              return OK;
                          }));
-    StopCtl done;
-    CILREG_TRY(ctl.finish(info, &done));
-    if (done.stop && ((nl - 1 - span_of_check(done.iters)) & 1))
-        CILREG_CUDA(cudaMemcpyAsync(u_out, ub[1], bytes, cudaMemcpyDeviceToDevice, s));
-    return OK;
+    if (checking && nl > 1) {
+        const SpanResult r = span_result(ub, nl, u_out);
+        CILREG_TRY(launch_take_span(ctl.ctl(), nl - 1, &r, 1, d.n, s));
+    }
+    return ctl.finish(info);
 }
 
 }  // namespace cilreg

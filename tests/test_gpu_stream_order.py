@@ -1,6 +1,7 @@
 """Stream order at both ends of a call.  The input may come from a kernel that
 has triggered its dependents (programmatic dependent launch) and still writes it
-when the call's first kernel starts."""
+when the call's first kernel starts; and a call that has returned has nothing
+left to write, so that its output may be read from any stream."""
 import ctypes
 import os
 import shutil
@@ -138,3 +139,45 @@ def test_prox_input_of_a_kernel_that_triggers_early(late_copy, monkeypatch, alg,
             assert C.cilreg_prox_session_destroy(h, s) == 0
     torch.cuda.synchronize()
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_nothing_is_left_to_write_when_a_stopped_call_returns(op):
+    """The rule fires at its fourth check (iteration 15) of 200 iterations; the
+    image is large enough for a late copy to be seen still running."""
+    import torch
+
+    f = torch.rand((8192, 8192), generator=torch.Generator("cuda").manual_seed(5), device="cuda")
+    call = _dev_calls()[op]
+    if op == "dtv":
+        call.ref = f.flip(0).contiguous()
+    out, info = torch.zeros_like(f), np.zeros(2, np.float32)
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    call(f, out, 200, 1e3, info, stream.cuda_stream)
+    done = stream.query()
+    with torch.cuda.stream(other):
+        seen = out.clone()
+    torch.cuda.synchronize()
+    assert int(info[0]) == 15
+    assert done and torch.equal(seen, out)
+
+
+@pytest.mark.parametrize("alg,prm,tol", [(1, [0.05, 0, 0], 1e3), (2, [0.05, 0], 1e3), (2, [0.05, 0], 0.0)])
+def test_nothing_is_left_to_write_when_a_prox_call_returns(alg, prm, tol):
+    import torch
+    from ccpi.filters.utils import cilregcuda as C
+
+    f = torch.rand((8192, 8192), generator=torch.Generator("cuda").manual_seed(5), device="cuda")
+    out, info = torch.zeros_like(f), (ctypes.c_float * 2)()
+    stream, h = torch.cuda.Stream(), ctypes.c_void_p()
+    ny, nx = f.shape
+    torch.cuda.synchronize()
+    s = stream.cuda_stream
+    assert C.cilreg_prox_session_create(ctypes.byref(h), alg, (ctypes.c_float * 4)(*prm), len(prm), nx, ny, 1, s) == 0
+    assert C.cilreg_prox_session_prox(h, f.data_ptr(), out.data_ptr(), 100, tol, info, s) == 0
+    done = stream.query()
+    torch.cuda.synchronize()
+    assert C.cilreg_prox_session_destroy(h, s) == 0
+    assert info[0] == (15 if tol else 100)
+    assert done
