@@ -6,7 +6,9 @@ return the list of results.  All volumes advance together on the GPU: one
 kernel launch per iteration covers the tiles of every volume and the whole
 iteration loop runs as one CUDA graph.  Each volume keeps its own stopping
 rule; results equal those of the single-volume calls (``regularisers.FGP_TV``,
-``regularisers.TGV``).
+``regularisers.TGV``): FGP's bit for bit where those all run one kernel family
+(images of even rows, images of odd rows, volumes below 2^21 voxels or of odd
+rows), else, and TGV's, to the last places.
 """
 from __future__ import annotations
 

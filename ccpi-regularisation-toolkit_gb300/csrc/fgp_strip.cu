@@ -1,6 +1,9 @@
 // FGP-TV and FGP-dTV on 2D images, several iterations per launch (strip2d.cuh),
-// with the arithmetic of k_fgp_x2_2d (FGP_TV_core.c:40-171, FGP_dTV_core.c:
-// 46-180), operation by operation.
+// operation by operation with the arithmetic of the kernel that runs such images
+// in a batch (FGP_TV_core.c:40-171, FGP_dTV_core.c:46-180): k_fgp_x2_2d's where
+// the rows are even, k_fgp_stream's where they are odd, so that a batch of either
+// equals its single calls bit for bit.  The two differ in which product of a sum
+// of two is rounded (dot2).
 //
 // A thread holds P^{k-1}, P^{k-2} and f (and b) of its rows: R takes the place
 // of P^{k-2} once it is formed, and P^{k-1} that of R once P^k is.  U of the
@@ -34,10 +37,17 @@ struct Args {
     bool nonneg, aniso, write_u;
 };
 
+// a1 b1 + a2 b2
+template <bool ODD>
+__device__ __forceinline__ float2 dot2(float2 a1, float2 b1, float2 a2, float2 b2) {
+    return ODD ? fma2(a1, b1, mul2(a2, b2)) : fma2(a2, b2, mul2(a1, b1));
+}
+
 // p scaled into the unit ball or clipped (utils.c:180-213)
+template <bool ODD>
 __device__ __forceinline__ void project(float2& p1, float2& p2, bool aniso) {
     if (!aniso) {
-        const float2 den = fma2(p2, p2, mul2(p1, p1));
+        const float2 den = dot2<ODD>(p1, p1, p2, p2);
         const float2 sq = make_float2((den.x > 1.f) ? rsqrt_normal(den.x) : 1.f,
                                       (den.y > 1.f) ? rsqrt_normal(den.y) : 1.f);
         p1 = mul2(p1, sq);
@@ -48,7 +58,7 @@ __device__ __forceinline__ void project(float2& p1, float2& p2, bool aniso) {
     }
 }
 
-template <int R, bool CHECK, bool DTV>
+template <int R, bool CHECK, bool DTV, bool ODD>
 __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
     k_fgp_strip2d(Args a, Frame fr) {
     __shared__ float2 first1[2][NW][32], first2[2][NW][32], last2[2][NW][32];
@@ -108,12 +118,12 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             }
             if (DTV) {
                 const float2 c1 = b1[DTV ? r : 0], c2 = b2[DTV ? r : 0];
-                const float2 ip = fma2(g2, c2, mul2(g1, c1));
+                const float2 ip = dot2<ODD>(g1, c1, g2, c2);
                 g1 = fma2(neg2(ip), c1, g1);
                 g2 = fma2(neg2(ip), c2, g2);
             }
             float2 n1 = fma2(mp2, g1, o1[r]), n2 = fma2(mp2, g2, o2[r]);
-            project(n1, n2, a.aniso);
+            project<ODD>(n1, n2, a.aniso);
             if (last && a.write_u) {
                 if (CHECK) add_norms(q, r, u, uo[CHECK ? r : 0][w][lane], pa, pb);
                 q.store(a.u, r, u);
@@ -133,7 +143,7 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             float2 r1 = fma2(cm, sub2(p1[r], o1[r]), p1[r]), r2 = fma2(cm, sub2(p2[r], o2[r]), p2[r]);
             if (DTV) {
                 const float2 c1 = b1[DTV ? r : 0], c2 = b2[DTV ? r : 0];
-                const float2 ip = fma2(r2, c2, mul2(r1, c1));
+                const float2 ip = dot2<ODD>(r1, c1, r2, c2);
                 r1 = fma2(neg2(ip), c1, r1);
                 r2 = fma2(neg2(ip), c2, r2);
             }
@@ -167,12 +177,16 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
     if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
 }
 
-using Kernel = decltype(&k_fgp_strip2d<2, false, false>);
-template <bool DTV>
-Kernel pick(int R, bool check) {
-    if (R == 2) return check ? k_fgp_strip2d<2, true, DTV> : k_fgp_strip2d<2, false, DTV>;
-    if (R == 3) return check ? k_fgp_strip2d<3, true, DTV> : k_fgp_strip2d<3, false, DTV>;
-    return check ? k_fgp_strip2d<4, true, DTV> : k_fgp_strip2d<4, false, DTV>;
+using Kernel = decltype(&k_fgp_strip2d<2, false, false, false>);
+template <bool DTV, bool ODD>
+Kernel pick_r(int R, bool check) {
+    if (R == 2) return check ? k_fgp_strip2d<2, true, DTV, ODD> : k_fgp_strip2d<2, false, DTV, ODD>;
+    if (R == 3) return check ? k_fgp_strip2d<3, true, DTV, ODD> : k_fgp_strip2d<3, false, DTV, ODD>;
+    return check ? k_fgp_strip2d<4, true, DTV, ODD> : k_fgp_strip2d<4, false, DTV, ODD>;
+}
+Kernel pick(int R, bool check, bool dtv, bool odd) {
+    if (odd) return dtv ? pick_r<true, true>(R, check) : pick_r<false, true>(R, check);
+    return dtv ? pick_r<true, false>(R, check) : pick_r<false, false>(R, check);
 }
 
 }  // namespace
@@ -237,7 +251,7 @@ int fgp_strip_run(const float* f, const float* const* b, float* u_out, float lam
         for (int t = 0; t < sp.count; t++) a.c[t] = cseq[sp.first + t];
         a.u = (checking && ((nl - 1 - k) & 1)) ? ualt : u_out;
         a.write_u = end || sp.check;
-        CILREG_CUDA(launch_strip(b ? pick<true>(P.R, checking) : pick<false>(P.R, checking), P, fr, checking, s, a));
+        CILREG_CUDA(launch_strip(pick(P.R, checking, b != nullptr, d.nx & 1), P, fr, checking, s, a));
         return OK;
     }));
     // what the check that fired, or the last launch, left: U, and a warm run's duals

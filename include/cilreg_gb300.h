@@ -181,7 +181,10 @@ int cilreg_tv_energy_dev(const float *d_u, const float *d_u0, float *E_val, floa
  * CILREG_BATCH_AUTOTUNE=1 times candidate z chunks of the FGP kernel on the
  * batch and keeps the choice, also in the file CILREG_AUTOTUNE_CACHE).  The
  * call returns when every output is written.  Results equal those of the
- * single-volume calls (FGP bit for bit, TGV to the last bits).
+ * single-volume calls: TGV to the last bits, FGP bit for bit where the single
+ * calls of all its volumes run one kernel family (images whose rows are all
+ * even or all odd; volumes each below 2^21 voxels or with odd rows), else
+ * within a few units in the last place.
  * ------------------------------------------------------------------------- */
 int cilreg_fgp_tv_batch_dev(int nvol, const float *const *d_in, float *const *d_out, const int *dims,
                             const float *lambdas, int iters, float epsil, int methodTV, int nonneg, float *infovectors,

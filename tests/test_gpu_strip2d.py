@@ -97,3 +97,32 @@ def test_strips_take_arrays_off_8_byte_alignment(monkeypatch, op):
     out, _ = _run(monkeypatch, "1", op, f, 17)
     ref, _ = _run(monkeypatch, "1", op, f.clone(), 17)
     np.testing.assert_array_equal(out, ref)
+
+
+@pytest.mark.parametrize("op", ["fgp0", "fgp1", "dtv0", "dtv1"])
+@pytest.mark.parametrize("shape", [(2, 3), (33, 63), (97, 131), (131, 127), (200, 319)])
+def test_strips_of_odd_rows_keep_the_streaming_kernels_bits(monkeypatch, op, shape):
+    f = _image(shape)
+    for tol in (0.0, 1e-7):
+        ref, _ = _run(monkeypatch, "0", op, f, 33, tol)
+        for plan in ("1",) + tuple(PLANS):
+            np.testing.assert_array_equal(_run(monkeypatch, plan, op, f, 33, tol)[0], ref, err_msg=plan)
+
+
+@pytest.mark.parametrize("shapes", [[(37, 51), (128, 9), (201, 199), (1, 77)], [(36, 52), (128, 10), (200, 200)]],
+                         ids=["odd rows", "even rows"])
+@pytest.mark.parametrize("epsil", [0.0, 3e-4])
+def test_fgp_batch_of_images_equals_single_calls(shapes, epsil):
+    """As they run by default: strips in a single call, the batch's own kernel in the batch."""
+    from ccpi.filters.batch import FGP_TV_batch
+    from ccpi.filters.regularisers import FGP_TV
+
+    rng = np.random.default_rng(5)
+    vols = [rng.random(s).astype(np.float32) for s in shapes]
+    lams = [0.03 + 0.01 * i for i in range(len(vols))]
+    infos = np.zeros((len(vols), 2), np.float32)
+    outs = FGP_TV_batch(vols, lams, 60, epsil, 0, 1, infovectors=infos)
+    for v, o, lam, inf in zip(vols, outs, lams, infos):
+        info = np.zeros(2, np.float32)
+        np.testing.assert_array_equal(o, FGP_TV(v, lam, 60, epsil, 0, 1, device="gpu", infovector=info))
+        assert int(inf[0]) == int(info[0])
