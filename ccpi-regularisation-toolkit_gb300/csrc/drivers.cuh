@@ -32,9 +32,8 @@ int rof_run(const float* f, float* u_out, const float* lam_arr, float lam, int i
 // One ROF iteration (the kernel rof_run launches) on caller-provided buffers:
 // reads `cur`, writes `nxt`; on a check iteration writes one FP64 partial per
 // CTA (num_blocks(plan_launch(d)) of them) for launch_finalize_check.
-// odd_pairs false: odd rows run one voxel per thread (the adjoint's states).
 int rof_launch_step(const float* cur, float* nxt, const float* f, const float* lam_arr, float lam, float tau,
-                    const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s, bool odd_pairs = true);
+                    const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s);
 // number of FP64 partial slots rof_launch_step writes on a check iteration
 long long rof_partial_slots(const Dims& d);
 // OK when the kernel rof_launch_step would run for `d` fits the launch grid

@@ -16,10 +16,11 @@
 //   Rbar_k = Qbar_k - lambda A^T Zbar_k,  (A^T Z)_c = Z - Z[+e_c] (0 past the last index)
 // One kernel per reverse iteration (k_adj_stream) forms Z_k, Qbar_k, Zbar_k
 // and Rbar_k of every volume of a batch of equal shapes.  The forward states
-// are stored every `ckpt` iterations and each segment is recomputed with the
-// production iteration kernel before its reverse sweep, so the linearisation
-// point is exactly the forward pass the caller saw; the last segment is
-// recomputed only, not run before as well.
+// are stored every `ckpt` iterations and each segment is recomputed before its
+// reverse sweep; the last segment is recomputed only, not run before as well.
+// They have k_fgp_stream's roundings: the bits of the forward pass that the
+// caller saw, except for images with even rows and for volumes with even rows
+// whose single call runs k_fgp_x2, which round a product or two otherwise.
 #include <math.h>
 
 #include <type_traits>

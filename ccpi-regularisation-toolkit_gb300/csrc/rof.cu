@@ -128,7 +128,7 @@ int rof_check_grid(const Dims& d) {
 }
 
 int rof_launch_step(const float* cur, float* nxt, const float* f, const float* lam_arr, float lam, float tau,
-                    const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s, bool odd_pairs) {
+                    const Dims& d, const StopCtl* ctl, int check, double2* partials, cudaStream_t s) {
     if (use_simple_kernel()) {
         const Launch3 L = plan_launch(d);
         if (d.nz > 1)
@@ -138,7 +138,7 @@ int rof_launch_step(const float* cur, float* nxt, const float* f, const float* l
                                                          partials);
         CILREG_CUDA(cudaGetLastError());
     } else {
-        CILREG_TRY(rof_tiled_step(rof_tiled_plan(d, odd_pairs), cur, nxt, f, lam_arr, lam, tau, d, ctl, check, partials, s));
+        CILREG_TRY(rof_tiled_step(rof_tiled_plan(d), cur, nxt, f, lam_arr, lam, tau, d, ctl, check, partials, s));
     }
     note_launch();
     return OK;

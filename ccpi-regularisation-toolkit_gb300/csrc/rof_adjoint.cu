@@ -25,8 +25,9 @@
 //   (J^T W)(v) = sum_c [ sum_{u : hi_c(u) = v} E_c(u) - E_c(v) + F_c(v) - sum_{u : lo_c(u) = v} F_c(u) ].
 // Two kernels per reverse iteration: coefficients (E, F and the lambda term)
 // and the gather.  The forward states are stored every `ckpt` iterations and
-// each segment is recomputed with the production iteration kernel, so the
-// linearisation point is exactly the forward pass the caller saw.
+// each segment is recomputed one iteration per launch (k_rof_pair in 3D, in 2D
+// the kernels whose bits the strips of a forward call keep), so the linearisation
+// point is exactly the forward pass the caller saw.
 #include <math.h>
 
 #include <vector>
@@ -213,15 +214,12 @@ int rof_vjp_run(const float* f, const float* ybar, float lam, int iters, float t
     CILREG_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), s));
     CILREG_CUDA(cudaMemsetAsync(fbar, 0, nb, s));
 
-    // The states run odd rows one voxel per thread: the two-voxel kernel rounds
-    // some sums otherwise, and the reverse sweep, discontinuous in the states,
-    // turns their last places into 1e-6 of the 64-bit lambda derivative.
     // pass 1: forward from f up to the last segment start, keeping U there
     // and at every earlier segment start
     const float* cur = f;
     for (int k = 0; k < (nseg - 1) * ckpt; k++) {
         float* nxt = ((k + 1) % ckpt == 0) ? ck[(k + 1) / ckpt] : ping[k & 1];
-        CILREG_TRY(rof_launch_step(cur, nxt, f, nullptr, lam, tau, d, ctl, 0, nullptr, s, false));
+        CILREG_TRY(rof_launch_step(cur, nxt, f, nullptr, lam, tau, d, ctl, 0, nullptr, s));
         cur = nxt;
     }
 
@@ -233,7 +231,7 @@ int rof_vjp_run(const float* f, const float* ybar, float lam, int iters, float t
         const float* start = (g == 0) ? f : ck[g];
         auto state = [&](int k) -> const float* { return (k == k0) ? start : seg[k - k0]; };
         for (int k = k0; k + 1 < k1; k++)
-            CILREG_TRY(rof_launch_step(state(k), seg[k + 1 - k0], f, nullptr, lam, tau, d, ctl, 0, nullptr, s, false));
+            CILREG_TRY(rof_launch_step(state(k), seg[k + 1 - k0], f, nullptr, lam, tau, d, ctl, 0, nullptr, s));
         for (int k = k1 - 1; k >= k0; k--) {
             RofAdjArgs a;
             a.u = state(k);

@@ -15,10 +15,9 @@
 // The j-axis neighbours of the pair are the pair's own other voxel and one
 // scalar load on each side.  Ring planes beyond the volume hold its mirrored
 // planes, so the k neighbours of the first and last plane need no select.
-// Per voxel this executes about 40% fewer instructions than k_rof_async; the
-// iterates agree with it to within a few units in the last place (the
-// one-voxel kernel's compiler-contracted multiply-adds are not all the ones
-// written out here).
+// Per voxel this executes about 40% fewer instructions than k_rof_async.  Odd
+// rows have its iterates bit for bit, even ones to within a few units in the
+// last place (they round one product of D3's sum first).
 //
 // A CTA of 16 x 16 threads holds a 32 x 16 tile with a one-voxel halo; the
 // inner 30 x 14 voxels are updated.  Tile x origins are even (x0 = 30 bx - 2)
@@ -55,11 +54,14 @@ struct Geo {
     static constexpr size_t SMEM = sizeof(float) * TP * (RING + 4);  // U ring, D1 and D2 (two planes each)
 };
 
-// square of minmod(a, b) per component (ROF_TV_core.c:132): the median of a,
-// b and 0 has its magnitude
+// minmod(a, b) per component up to its sign (ROF_TV_core.c:132): the median of
+// a, b and 0 has its magnitude; and its square
+__device__ __forceinline__ float2 minmod2(float2 a, float2 b) {
+    return make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
+                       fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
+}
 __device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
-    const float2 m = make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
-                                 fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
+    const float2 m = minmod2(a, b);
     return mul2(m, m);
 }
 
@@ -71,7 +73,8 @@ __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
-template <bool CHECK, bool LARR, bool ALIGNED, int ROWS, bool LATE>
+// ODD: rows of odd length (not ALIGNED)
+template <bool CHECK, bool LARR, bool ALIGNED, int ROWS, bool LATE, bool ODD = false>
 __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
     k_rof_pair(const float* __restrict__ U, float* __restrict__ Un, const float* __restrict__ F,
                const float* __restrict__ lam_arr, float lam, float tau, Dims d, int zc, const StopCtl* ctl,
@@ -156,10 +159,17 @@ __global__ void __launch_bounds__(Geo<ROWS>::NTP, Geo<ROWS>::MINB)
         const float2 xm = make_float2(ub.x - Um[oxl], dxc);
         const float2 yp = sub2(ld2(Um + oyh), ub), ym = sub2(ub, ld2(Um + oyl));
         const float2 zp = sub2(uc, ub), zm = sub2(ub, ua);
-        const float2 mx2 = minmod_sq2(xp, xm), my2 = minmod_sq2(yp, ym), mz2 = minmod_sq2(zp, zm);
-        const float2 n1 = normalise2(yp, add2(add2(fma2(yp, yp, mx2), mz2), EPS2));
-        const float2 n2 = normalise2(xp, add2(add2(fma2(xp, xp, my2), mz2), EPS2));
-        const float2 n3 = normalise2(zp, add2(add2(fma2(zp, zp, my2), mx2), EPS2));
+        // the second minmod's square joins by a multiply-add, but for D3's in even
+        // rows, whose product is rounded first: odd rows have k_rof_async's
+        // iterates bit for bit, which the adjoint (discontinuous in the states:
+        // other last places move the lambda derivative by 1e-6) and its forward
+        // pass share
+        const float2 mx = minmod2(xp, xm), my = minmod2(yp, ym), mz = minmod2(zp, zm);
+        const float2 mx2 = mul2(mx, mx), my2 = mul2(my, my);
+        const float2 n1 = normalise2(yp, add2(fma2(mz, mz, fma2(yp, yp, mx2)), EPS2));
+        const float2 n2 = normalise2(xp, add2(fma2(mz, mz, fma2(xp, xp, my2)), EPS2));
+        const float2 s3 = fma2(zp, zp, my2);
+        const float2 n3 = normalise2(zp, add2(ODD ? fma2(mx, mx, s3) : add2(s3, mx2), EPS2));
         st2(sD1 + (1 - P) * TP + o, n1);
         st2(sD2 + (1 - P) * TP + o, n2);
         // C. update plane j-2 (ROF_TV_core.c:269-297): lower fluxes D1(i-1)
@@ -293,20 +303,25 @@ __global__ void __launch_bounds__(NTP2, 8)
 constexpr int ROWS = 16;
 using PairKernel = decltype(&k_rof_pair<false, false, true, ROWS, true>);
 
+enum Form { FORM_ALIGNED, FORM_SHIFTED, FORM_ODD };  // even rows, 8-byte aligned or not; odd rows
+
+template <bool LATE, bool ALIGNED, bool ODD>
+PairKernel pick_t(bool check, bool larr) {
+    return check ? (larr ? k_rof_pair<true, true, ALIGNED, ROWS, LATE, ODD> : k_rof_pair<true, false, ALIGNED, ROWS, LATE, ODD>)
+                 : (larr ? k_rof_pair<false, true, ALIGNED, ROWS, LATE, ODD> : k_rof_pair<false, false, ALIGNED, ROWS, LATE, ODD>);
+}
 template <bool LATE>
-PairKernel pick_t(bool check, bool larr, bool aligned) {
-    if (aligned)
-        return check ? (larr ? k_rof_pair<true, true, true, ROWS, LATE> : k_rof_pair<true, false, true, ROWS, LATE>)
-                     : (larr ? k_rof_pair<false, true, true, ROWS, LATE> : k_rof_pair<false, false, true, ROWS, LATE>);
-    return check ? (larr ? k_rof_pair<true, true, false, ROWS, LATE> : k_rof_pair<true, false, false, ROWS, LATE>)
-                 : (larr ? k_rof_pair<false, true, false, ROWS, LATE> : k_rof_pair<false, false, false, ROWS, LATE>);
+PairKernel pick_f(bool check, bool larr, Form form) {
+    return form == FORM_ALIGNED   ? pick_t<LATE, true, false>(check, larr)
+           : form == FORM_SHIFTED ? pick_t<LATE, false, false>(check, larr)
+                                  : pick_t<LATE, false, true>(check, larr);
 }
 // late: where the kernel triggers its successor (pdl_many_waves), chosen here
 // at compile time (the late trigger's code costs the early variant 2%): late
 // for a grid of one wave, four CTAs per SM (192^3 32.8 -> 31.0 us per
 // iteration), early above (256^3 62.8 against 63.6)
-PairKernel pick(bool check, bool larr, bool aligned, bool late) {
-    return late ? pick_t<true>(check, larr, aligned) : pick_t<false>(check, larr, aligned);
+PairKernel pick(bool check, bool larr, Form form, bool late) {
+    return late ? pick_f<true>(check, larr, form) : pick_f<false>(check, larr, form);
 }
 
 PairKernel pick2d(bool check, bool larr, bool aligned) {
@@ -323,8 +338,8 @@ bool smem_ready() {
         bool r = true;
         for (int c = 0; c < 2; c++)
             for (int l = 0; l < 2; l++)
-                for (int a = 0; a < 4; a++)
-                    r = r && cudaFuncSetAttribute(pick(c, l, a & 1, a & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                for (int a = 0; a < 6; a++)
+                    r = r && cudaFuncSetAttribute(pick(c, l, Form(a % 3), a / 3), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)Geo<ROWS>::SMEM) == cudaSuccess;
         cudaGetLastError();
         return r;
@@ -373,9 +388,10 @@ int rof_pair_step(const RofPlan& T, const float* cur, float* nxt, const float* f
                                tau, d, 1, ctl, partials));
         return OK;
     }
+    const Form form = aligned ? FORM_ALIGNED : d.nx % 2 == 0 ? FORM_SHIFTED : FORM_ODD;
     if (!smem_ready())
         return fail(ERR_CUDA, __FILE__, __LINE__, "cannot raise the shared-memory limit of k_rof_pair");
-    CILREG_CUDA(launch_pdl(pick(check != 0, larr, aligned, T.nblocks <= 4LL * sm_count()), T.grid, T.block, Geo<ROWS>::SMEM, s, cur, nxt, f,
+    CILREG_CUDA(launch_pdl(pick(check != 0, larr, form, T.nblocks <= 4LL * sm_count()), T.grid, T.block, Geo<ROWS>::SMEM, s, cur, nxt, f,
                            lam_arr, lam, tau, d, T.zchunk, ctl, partials));
     return OK;
 }

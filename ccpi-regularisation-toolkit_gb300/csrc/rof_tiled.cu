@@ -489,8 +489,8 @@ int rof_tb2d_step(const float* cur, float* nxt, const float* f, const float* lam
     return OK;
 }
 
-RofPlan rof_tiled_plan(const Dims& d, bool odd_pairs) {
-    if (rof_pair_applies(d) && (odd_pairs || d.nx % 2 == 0)) return rof_pair_plan(d);
+RofPlan rof_tiled_plan(const Dims& d) {
+    if (rof_pair_applies(d)) return rof_pair_plan(d);
     RofPlan T;
     T.block = dim3(BX, BY, 1);
     const long long tiles = (long long)((d.nx + OX - 1) / OX) * ((d.ny + OY - 1) / OY);

@@ -12,8 +12,7 @@ struct RofPlan {
     bool pair = false;  // the two-voxels-per-thread kernel (rof_pair.cu)
 };
 
-// odd_pairs: volumes with odd rows run the two-voxel kernel too
-RofPlan rof_tiled_plan(const Dims& d, bool odd_pairs = true);
+RofPlan rof_tiled_plan(const Dims& d);
 
 // volumes of fewer than 2^31 voxels run k_rof_pair; of 2D images those with nx
 // even that do not run strips run k_rof_pair2d (CILREG_ROF_KERNEL=async, reg or

@@ -815,3 +815,30 @@ def test_fgp_shuffle_kernel_matches_the_one_voxel_kernel(method, shape, monkeypa
             want = R.FGP_TV(x, 0.05, 70, tol, method, nonneg).cpu().numpy()
             monkeypatch.delenv("CILREG_FGP_KERNEL")
             np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 3), (5, 16, 29), (9, 30, 31), (7, 15, 61), (70, 29, 57), (3, 1, 5)])
+@pytest.mark.parametrize("lam_map", [False, True])
+def test_rof_odd_rows_keep_the_one_voxel_kernels_bits(lam_map, shape, monkeypatch):
+    """3D ROF volumes with odd rows: the two-voxel kernel and the one-voxel one
+    agree bit for bit, so the adjoint's states are the forward pass whichever runs."""
+    import torch
+    from ccpi.filters.utils import cilregcuda as C
+
+    rng = np.random.default_rng(12)
+    x = torch.from_numpy((rng.random(shape) + np.arange(shape[-1]) // 5 % 2).astype(np.float32)).cuda()
+    lam = torch.from_numpy(rng.uniform(0.1, 0.9, shape).astype(np.float32)).cuda()
+    torch.cuda.synchronize()
+
+    def run(tol):
+        out = torch.zeros_like(x)
+        assert C.cilreg_rof_tv_dev(x.data_ptr(), out.data_ptr(), None, lam.data_ptr() if lam_map else None, 0.7, 22, 0.1,
+                                   tol, *shape[::-1], torch.cuda.current_stream().cuda_stream) == 0
+        return out.cpu().numpy()
+
+    for tol in (0.0, 1e-7):
+        got = run(tol)
+        monkeypatch.setenv("CILREG_ROF_KERNEL", "async")
+        want = run(tol)
+        monkeypatch.delenv("CILREG_ROF_KERNEL")
+        np.testing.assert_array_equal(got, want)

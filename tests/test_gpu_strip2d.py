@@ -99,7 +99,7 @@ def test_strips_take_arrays_off_8_byte_alignment(monkeypatch, op):
     np.testing.assert_array_equal(out, ref)
 
 
-@pytest.mark.parametrize("op", ["fgp0", "fgp1", "dtv0", "dtv1"])
+@pytest.mark.parametrize("op", ["fgp0", "fgp1", "dtv0", "dtv1", "rof"])
 @pytest.mark.parametrize("shape", [(2, 3), (33, 63), (97, 131), (131, 127), (200, 319)])
 def test_strips_of_odd_rows_keep_the_streaming_kernels_bits(monkeypatch, op, shape):
     f = _image(shape)
