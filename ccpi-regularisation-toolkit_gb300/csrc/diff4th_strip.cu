@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
     struct Row {
         float2 c, lo, hi;  // the pair, (x-1, x) and (x+1, x+2)
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
             c = next;
         }
     };
-    auto update = [&](auto edge_, float2 wm, float2 wbelow, bool sum) {
+    auto update = [&](auto edge_, float2 wm, float2 wbelow, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -77,12 +77,12 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
             const float2 ly = fma2(MTWO2, wc, add2(wm, wh));
             const float2 lap = add2(lx, ly);
             const float2 un = fma2(tau2, fma2(mlam2, lap, neg2(sub2(u[r], f[r]))), u[r]);
-            if (CHECK && sum) add_norms(q, r, un, u[r], pa, pb);
+            if (CHECK && sum) add_norms(q, r, un, u[r], norms);
             u[r] = un;
             wm = W[r];
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         firstU[w][lane] = u[0];
         lastU[w][lane] = u[R - 1];
         __syncthreads();
@@ -98,13 +98,13 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
         const float2 wbelow = w < NW - 1 ? firstW[w + 1][lane] : W[R - 1];
         const float2 wabove = q.Y == 0 ? W[1] : (w > 0 ? lastW[w - 1][lane] : W[0]);
         if (q.edge)
-            update(std::true_type{}, wabove, wbelow, t == fr.count - 1);
+            update(std::true_type{}, wabove, wbelow, sum);
         else
-            update(std::false_type{}, wabove, wbelow, t == fr.count - 1);
-    }
+            update(std::false_type{}, wabove, wbelow, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_d4_strip2d<2, false>);

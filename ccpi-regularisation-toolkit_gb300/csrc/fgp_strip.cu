@@ -88,9 +88,9 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
     }
     const float2 mlam2 = splat(-a.lam), mp2 = splat(a.multip);
     const bool top = q.Y == 0;
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
-    auto iterate = [&](auto edge_, float2 r2up, float2 r1dn, float2 r2dn, int t) {
+    auto iterate = [&](auto edge_, float2 r2up, float2 r1dn, float2 r2dn, int t, auto last) {
         constexpr bool EDGE = decltype(edge_)::value;
         // U = f - lambda div R, zero flux below index 0 (FGP_TV_core.c:220-236)
         auto u_of = [&](float2 r1, float2 r2, float2 r2above, float2 fv) -> float2 {
@@ -101,7 +101,6 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             if (a.nonneg) u = make_float2(u.x < 0.f ? 0.f : u.x, u.y < 0.f ? 0.f : u.y);
             return u;
         };
-        const bool last = t == fr.count - 1;
         float2 u = u_of(o1[0], o2[0], r2up, f[0]);
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -125,7 +124,7 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             float2 n1 = fma2(mp2, g1, o1[r]), n2 = fma2(mp2, g2, o2[r]);
             project<ODD>(n1, n2, a.aniso);
             if (last && a.write_u) {
-                if (CHECK) add_norms(q, r, u, uo[CHECK ? r : 0][w][lane], pa, pb);
+                if (CHECK) add_norms(q, r, u, uo[CHECK ? r : 0][w][lane], norms);
                 q.store(a.u, r, u);
             }
             if (CHECK && t == fr.count - 2) uo[CHECK ? r : 0][w][lane] = u;
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             u = un;
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto last) {
         const float2 cm = splat(a.c[t]);
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -159,10 +158,10 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
         const float2 r1dn = w < NW - 1 ? first1[s][w + 1][lane] : o1[R - 1];
         const float2 r2dn = w < NW - 1 ? first2[s][w + 1][lane] : o2[R - 1];
         if (q.edge)
-            iterate(std::true_type{}, r2up, r1dn, r2dn, t);
+            iterate(std::true_type{}, r2up, r1dn, r2dn, t, last);
         else
-            iterate(std::false_type{}, r2up, r1dn, r2dn, t);
-    }
+            iterate(std::false_type{}, r2up, r1dn, r2dn, t, last);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) {
         if (a.qc[0]) {
@@ -174,7 +173,7 @@ __global__ void __launch_bounds__(NT, R <= 2 || (R == 3 && !DTV) ? 2 : 1)
             q.store(a.qo[1], r, o2[r]);
         }
     }
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_fgp_strip2d<2, false, false, false>);

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     if (!begin<CHECK>(fr)) return;
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
     auto sign_terms = [](float2 v1, float2 v2, float2& t1, float2& t2) {
         t1 = llt_sign2(v1);
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
     // row -1 is the mirrored row 1 at the image's first row: `above`, with its
     // own upper and lower rows above_h and above_l; below2 is the row under
     // the row under the strip
-    auto iterate = [&](auto edge_, float2 above_l, float2 above, float2 above_h, float2 below, float2 below2, bool sum) {
+    auto iterate = [&](auto edge_, float2 above_l, float2 above, float2 above_h, float2 below, float2 below2, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
         float2 r1l, l2l;  // R1 and L2 of the row above
         {
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
                 const float2 g = odd ? fma2(lrof2, div, mul2(mlllt2, lap)) : fma2(mlllt2, lap, mul2(lrof2, div));
                 const float2 t = sub2(g, sub2(um, f[k]));
                 const float2 un = fma2(tau2, t, um);
-                if (CHECK && sum) add_norms(q, k, un, um, pa, pb);
+                if (CHECK && sum) add_norms(q, k, un, um, norms);
                 u[k] = un;
                 r1l = r1;
                 l2l = l2;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
             um = c;
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         const int b = t & 1;
         first[b][0][w][lane] = u[0];
         first[b][1][w][lane] = u[1];
@@ -124,13 +124,13 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1)
         const float2 above_l = top ? u[0] : (w > 0 ? last[b][1][w - 1][lane] : u[0]);
         const float2 above_h = top ? (q.ny == 2 ? u[0] : (R > 2 ? u[R > 2 ? 2 : 0] : below)) : u[0];
         if (q.edge)
-            iterate(std::true_type{}, above_l, above, above_h, below, below2, t == fr.count - 1);
+            iterate(std::true_type{}, above_l, above, above_h, below, below2, sum);
         else
-            iterate(std::false_type{}, above_l, above, above_h, below, below2, t == fr.count - 1);
-    }
+            iterate(std::false_type{}, above_l, above, above_h, below, below2, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_llt_strip2d<2, false>);

@@ -26,9 +26,9 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     const float2 isg2 = splat(isg), lam2 = splat(lam), tau2 = splat(tau);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
-    auto iterate = [&](auto edge_, float2 above, float2 below, bool sum) {
+    auto iterate = [&](auto edge_, float2 above, float2 below, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
         float2 south = flux2<PEN>(sub2(u[0], above), sg, isg2);
 #pragma unroll
@@ -45,12 +45,12 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
             const float2 s = sub2(add2(sub2(fx, make_float2(west, fx.x)), fy), south);
             const float2 t = sub2(c, f[r]);
             const float2 un = fma2(tau2, fma2(lam2, s, neg2(t)), c);
-            if (CHECK && sum) add_norms(q, r, un, c, pa, pb);
+            if (CHECK && sum) add_norms(q, r, un, c, norms);
             u[r] = un;
             south = fy;
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         const int b = t & 1;
         first[b][w][lane] = u[0];
         last[b][w][lane] = u[R - 1];
@@ -58,13 +58,13 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         const float2 below = w < NW - 1 ? first[b][w + 1][lane] : u[R - 1];
         const float2 above = q.Y == 0 ? u[1] : (w > 0 ? last[b][w - 1][lane] : u[0]);
         if (q.edge)
-            iterate(std::true_type{}, above, below, t == fr.count - 1);
+            iterate(std::true_type{}, above, below, sum);
         else
-            iterate(std::false_type{}, above, below, t == fr.count - 1);
-    }
+            iterate(std::false_type{}, above, below, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_ndf_strip2d<0, 2, false>);

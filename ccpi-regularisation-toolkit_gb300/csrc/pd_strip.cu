@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
         p2[r] = a.p[0] ? q.load(a.p[1], r) : splat(0.f);
     }
     const float2 sigma2 = splat(a.sigma), tau2 = splat(a.tau);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
     // P += sigma grad U, projected (mirrored differences at the far edges)
     auto dual = [&](auto edge_, float2 above, float2 below) {
@@ -90,9 +90,8 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
             um = u[r];
         }
     };
-    auto primal = [&](auto edge_, float2 p2up, int t) {
+    auto primal = [&](auto edge_, float2 p2up, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
-        const bool sum = CHECK && t == fr.count - 1;
 #pragma unroll
         for (int r = 0; r < R; r++) {
             float lo = left_of(p1[r]);
@@ -103,14 +102,14 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
             if (a.nonneg) uc = make_float2(uc.x < 0.f ? 0.f : uc.x, uc.y < 0.f ? 0.f : uc.y);
             const float2 un = div2(add2(sub2(uc, mul2_rn(tau2, dv)), ltf[r]), a.onelt);
             if (CHECK && sum) {
-                add_norms(q, r, un, uc, pa, pb);
+                add_norms(q, r, un, uc, norms);
                 q.store(a.brk, r, un);
             }
             u[r] = add2(un, sub2(un, uc));  // theta = 1
             p2up = p2[r];
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         firstU[w][lane] = u[0];
         lastU[w][lane] = u[R - 1];
         __syncthreads();
@@ -124,10 +123,10 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
         __syncthreads();
         const float2 p2up = q.Y == 0 ? splat(0.f) : (w > 0 ? lastP[w - 1][lane] : p2[0]);
         if (q.edge)
-            primal(std::true_type{}, p2up, t);
+            primal(std::true_type{}, p2up, sum);
         else
-            primal(std::false_type{}, p2up, t);
-    }
+            primal(std::false_type{}, p2up, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) {
         q.store(a.un, r, u[r]);
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
             q.store(a.pn[1], r, p2[r]);
         }
     }
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_pd_strip2d<2, false>);

@@ -47,11 +47,11 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
 #pragma unroll
     for (int r = 0; r < R; r++) u[r] = q.load(U, r);
     const float2 EPS2 = splat(1.0e-8f), tau2 = splat(tau);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
     // above: the row over the strip (the mirrored row 1 over row 0), next: the
     // row under that one
-    auto iterate = [&](auto edge_, float2 above, float2 next, float2 below, bool sum) {
+    auto iterate = [&](auto edge_, float2 above, float2 next, float2 below, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
         // squared minmod of the x differences of a row, and its forward difference
         auto along_x = [&](float2& c, float2& xp, float2& mx2) {
@@ -85,13 +85,13 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
             const float2 div = add2(sub2(d1, d1l), sub2(d2, make_float2(d2l, d2.x)));
             const float2 t = sub2(c, f[r]);
             const float2 un = fma2(tau2, fma2(l[LARR ? r : 0], div, neg2(t)), c);
-            if (CHECK && sum) add_norms(q, r, un, c, pa, pb);
+            if (CHECK && sum) add_norms(q, r, un, c, norms);
             u[r] = un;
             ym = yp;
             d1l = d1;
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         const int b = t & 1;
         first[b][w][lane] = u[0];
         last[b][w][lane] = u[R - 1];
@@ -100,13 +100,13 @@ __global__ void __launch_bounds__(NT, R <= 4 ? 2 : 1)
         const float2 above = Y == 0 ? u[1] : (w > 0 ? last[b][w - 1][lane] : u[0]);
         const float2 next = Y == 0 ? (R > 2 ? u[R > 2 ? 2 : 0] : below) : u[0];
         if (q.edge)
-            iterate(std::true_type{}, above, q.ny == 2 && Y == 0 ? u[0] : next, below, t == fr.count - 1);
+            iterate(std::true_type{}, above, q.ny == 2 && Y == 0 ? u[0] : next, below, sum);
         else
-            iterate(std::false_type{}, above, next, below, t == fr.count - 1);
-    }
+            iterate(std::false_type{}, above, next, below, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) q.store(Un, r, u[r]);
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_rof_strip2d<2, false, false>);

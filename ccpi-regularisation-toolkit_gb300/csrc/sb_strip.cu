@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
         q2up = sub2(q.load(a.d0[1], up), q.load(a.bp[1], up));
     }
     const float2 lam2 = splat(a.lambda), norm2 = splat(a.norm);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
     float2 g[R], u1[R];
 
     auto sum4 = [](float2 xh, float2 xl, float2 yh, float2 yl) { return add2(add2(add2(xh, xl), yh), yl); };
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
             ql = q2[r];
         }
     };
-    auto sweep2 = [&](auto edge_, float2 above, float2 below, bool sum) {
+    auto sweep2 = [&](auto edge_, float2 above, float2 below, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
         float2 um = above;
 #pragma unroll
@@ -126,12 +126,12 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
             if (EDGE && r == q.bottom) uh = um;
             const float2 s = add2(g[r], sum4(make_float2(c.y, hi), make_float2(lo, c.x), uh, um));
             const float2 un = mul2(norm2, fma2(s, lam2, muf[r]));
-            if (CHECK && sum) add_norms(q, r, un, u1[r], pa, pb);
+            if (CHECK && sum) add_norms(q, r, un, u1[r], norms);
             u[r] = un;
             um = u1[r];
         }
     };
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         firstU[w][lane] = u[0];
         lastU[w][lane] = u[R - 1];
         lastB1[w][lane] = b1[R - 1];
@@ -153,10 +153,10 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
         const float2 below1 = w < NW - 1 ? first1[w + 1][lane] : u1[R - 1];
         const float2 above1 = top ? u1[1] : (w > 0 ? last1[w - 1][lane] : u1[0]);
         if (q.edge)
-            sweep2(std::true_type{}, above1, below1, t == fr.count - 1);
+            sweep2(std::true_type{}, above1, below1, sum);
         else
-            sweep2(std::false_type{}, above1, below1, t == fr.count - 1);
-    }
+            sweep2(std::false_type{}, above1, below1, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) {
         q.store(a.un, r, u[r]);
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(NT, R <= 2 ? 2 : 1) k_sb_strip2d(Args a, Frame
             q.store(a.bn[1], r, b2[r]);
         }
     }
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_sb_strip2d<2, false>);

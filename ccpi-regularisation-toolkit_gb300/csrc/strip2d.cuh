@@ -23,6 +23,8 @@
 // axis have no halo on that side.
 #pragma once
 
+#include <float.h>
+
 #include "drivers.cuh"
 #include "pair.cuh"
 
@@ -157,18 +159,41 @@ cudaError_t launch_strip(Kernel kernel, const Plan& P, const Frame& F, bool rule
     const dim3 grid = rule ? dim3((unsigned)(P.nblocks + (F.check.n > 0 ? 1 : 0))) : dim3((unsigned)P.gx, (unsigned)P.gy);
     return launch_chained(F.follows, kernel, grid, dim3(32, NW, 1), 0, s, args..., F);
 }
-// one FP64 partial of the CTA's FP32 sums.  Two warps add the threads' sums
-// from shared memory: the FP64 unit takes 16 cycles for a warp's addition, and
-// a shuffle reduction of both sums in every warp is 170 of them per CTA
-// against 42.
-__device__ __forceinline__ void store_partial(float a, float b, double2* slot) {
-    __shared__ float sum[2][NT];
+// A thread's sums of a check over its rows: squared change (x) and square (y),
+// each as an FP32 sum and its rounding error, so that a thread's rows lose
+// nothing to each other.  (FP64 sums instead would be 2 R additions in every
+// warp, 16 cycles each.)  The two sums issue paired.
+struct Norms {
+    float2 s = make_float2(0.f, 0.f), e = make_float2(0.f, 0.f);
+};
+__device__ __forceinline__ void add_exact(Norms& n, float2 x) {
+    const float2 t = add2(n.s, x), v = sub2(t, n.s);
+    n.e = add2(n.e, add2(sub2(n.s, sub2(t, v)), sub2(x, v)));
+    n.s = t;
+}
+
+// One FP64 partial of the CTA's sums.  Two warps add the threads' sums from
+// shared memory: the FP64 unit takes 16 cycles for a warp's addition, and a
+// shuffle reduction of both sums in every warp is 170 of them per CTA against
+// 44.  The errors, 2^-24 of the sums, are added in FP32.
+__device__ __forceinline__ void store_partial(const Norms& n, double2* slot) {
+    __shared__ float sum[2][NT], err[2][NW];
     const int lane = threadIdx.x, w = threadIdx.y;
-    sum[0][w * 32 + lane] = a;
-    sum[1][w * 32 + lane] = b;
+    sum[0][w * 32 + lane] = n.s.x;
+    sum[1][w * 32 + lane] = n.s.y;
+    float ea = fabsf(n.e.x) <= FLT_MAX ? n.e.x : 0.f, eb = fabsf(n.e.y) <= FLT_MAX ? n.e.y : 0.f;  // an infinite sum has none
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ea += __shfl_down_sync(0xffffffffu, ea, o);
+        eb += __shfl_down_sync(0xffffffffu, eb, o);
+    }
+    if (lane == 0) {
+        err[0][w] = ea;
+        err[1][w] = eb;
+    }
     __syncthreads();
     if (w < 2) {
-        double v = 0.0;
+        double v = lane < NW ? (double)err[w][lane] : 0.0;
 #pragma unroll
         for (int j = 0; j < NW; j++) v += (double)sum[w][j * 32 + lane];
         v = warp_sum(v);
@@ -292,15 +317,39 @@ __device__ __forceinline__ void x_neighbours(const Place<R>& q, float2& v, float
     }
 }
 
+// A launch's iterations: pass(t, last).  With a rule the last one, whose change a
+// check sums, is a copy of its own, so that the sums take no registers before it
+// (a type, not a bool, as `last`).
+template <bool B>
+struct Flag {
+    __device__ constexpr operator bool() const { return B; }
+};
+template <bool CHECK, class Pass>
+__device__ __forceinline__ void iterations(int count, Pass pass) {
+    if constexpr (CHECK) {
+        for (int t = 0; t < count - 1; t++) pass(t, Flag<false>{});
+        pass(count - 1, Flag<true>{});
+    } else {
+        for (int t = 0; t < count; t++) pass(t, t == count - 1);
+    }
+}
+
 // adds the stored pixels' squared change and square of one row
 template <int R>
-__device__ __forceinline__ void add_norms(const Place<R>& q, int r, float2 un, float2 u, float2& pa, float2& pb) {
+__device__ __forceinline__ void add_norms(const Place<R>& q, int r, float2 un, float2 u, Norms& n) {
     if (q.Y + r < q.y0 || q.Y + r >= q.y1) return;
     const float2 df = sub2(un, u);
     const float2 dm = make_float2(q.vx ? df.x : 0.f, q.vy ? df.y : 0.f);
     const float2 um = make_float2(q.vx ? un.x : 0.f, q.vy ? un.y : 0.f);
-    pa = fma2(dm, dm, pa);
-    pb = fma2(um, um, pb);
+    // as the kernels of one iteration per launch: a pixel pair of even rows summed
+    // in FP32, every pixel of odd rows by itself
+    const float2 x = make_float2(dm.x, um.x), y = make_float2(dm.y, um.y);
+    if (q.nx & 1) {
+        add_exact(n, mul2_rn(x, x));
+        add_exact(n, mul2_rn(y, y));
+    } else {
+        add_exact(n, fma2(y, y, mul2_rn(x, x)));
+    }
 }
 
 // The launches of a run: each(k, span, frame) enqueues launch k.  The check of

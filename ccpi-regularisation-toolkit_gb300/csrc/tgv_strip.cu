@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
     }
     const float2 tau2 = splat(a.tau), lam2 = splat(a.lambda), ilt2 = splat(a.inv_lt), HALF2 = splat(0.5f),
                  TWO2 = splat(2.f);
-    float2 pa = splat(0.f), pb = splat(0.f);
+    Norms norms;
 
     // P and Q (sigma == tau)
     auto dual = [&](auto edge_, float2 ub, float2 v1b, float2 v2b) {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
         }
     };
     // U and V; (p2u, q2u, q3u): P2, Q2, Q3 of the row above
-    auto primal = [&](auto edge_, float2 p2u, float2 q2u, float2 q3u, bool sum) {
+    auto primal = [&](auto edge_, float2 p2u, float2 q2u, float2 q3u, auto sum) {
         constexpr bool EDGE = decltype(edge_)::value;
         // backward differences: X at index 0, -X[-1] at the last (TGV_core.c:286-292)
         auto back_x = [&](float2 c) {
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
             const float2 dv = add2(back_x(p1[r]), back_y(p2[r], p2u));
             const float2 un = mul2(fma2(lam2, fma2(tau2, dv, u[r]), tf[r]), ilt2);
             const float2 ue = fma2(TWO2, un, neg2(u[r]));
-            if (CHECK && sum) add_norms(q, r, ue, u[r], pa, pb);
+            if (CHECK && sum) add_norms(q, r, ue, u[r], norms);
             u[r] = ue;
             // UpdV_2D + newV (TGV_core.c:308-345)
             const float2 d1 = add2(back_x(q1[r]), back_y(q3[r], q3u));
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
         }
     };
     const bool top = q.Y == 0;
-    for (int t = 0; t < fr.count; t++) {
+    iterations<CHECK>(fr.count, [&](int t, auto sum) {
         firstUV[0][w][lane] = u[0];
         firstUV[1][w][lane] = v1[0];
         firstUV[2][w][lane] = v2[0];
@@ -160,10 +160,10 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
         const float2 p2u = top ? splat(0.f) : lastPQ[0][wa][lane], q2u = top ? splat(0.f) : lastPQ[1][wa][lane],
                      q3u = top ? splat(0.f) : lastPQ[2][wa][lane];
         if (q.edge)
-            primal(std::true_type{}, p2u, q2u, q3u, t == fr.count - 1);
+            primal(std::true_type{}, p2u, q2u, q3u, sum);
         else
-            primal(std::false_type{}, p2u, q2u, q3u, t == fr.count - 1);
-    }
+            primal(std::false_type{}, p2u, q2u, q3u, sum);
+    });
 #pragma unroll
     for (int r = 0; r < R; r++) {
         q.store(a.un, r, u[r]);
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(NT, 1) k_tgv_strip2d(Args a, Frame fr) {
             q.store(a.sn[6], r, q3[r]);
         }
     }
-    if (CHECK) store_partial(pa.x + pa.y, pb.x + pb.y, fr.partials + tile_index<CHECK>(fr));
+    if (CHECK) store_partial(norms, fr.partials + tile_index<CHECK>(fr));
 }
 
 using Kernel = decltype(&k_tgv_strip2d<2, false>);

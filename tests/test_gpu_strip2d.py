@@ -126,3 +126,28 @@ def test_fgp_batch_of_images_equals_single_calls(shapes, epsil):
         info = np.zeros(2, np.float32)
         np.testing.assert_array_equal(o, FGP_TV(v, lam, 60, epsil, 0, 1, device="gpu", infovector=info))
         assert int(inf[0]) == int(info[0])
+
+
+@pytest.mark.parametrize("width", [64, 63])
+@pytest.mark.parametrize("step", [1.0, 3.0])
+def test_check_sums_lose_nothing_to_a_threads_other_rows(monkeypatch, width, step):
+    """FGP's first iteration leaves U = f, so the check's relative change is known
+    from f and the output's initial content.  Every fourth row's squares are 2^24
+    times the others': one FP32 sum over a thread's four rows would lose those."""
+    import ctypes
+
+    import torch
+    from ccpi.filters.utils import cilregcuda as C
+
+    monkeypatch.setenv("CILREG_STRIP2D", "4,5")
+    f = np.ones((64, width), np.float32)
+    f[::4] = 4096.0
+    prev = f - np.float32(step)
+    d_f, d_u = torch.from_numpy(f).cuda(), torch.from_numpy(prev).cuda()
+    info = (ctypes.c_float * 2)()
+    assert C.cilreg_fgp_tv_dev(d_f.data_ptr(), d_u.data_ptr(), info, 0.05, 1, 1e-9, 0, 0, width, 64, 1,
+                               torch.cuda.current_stream().cuda_stream) == 0
+    np.testing.assert_array_equal(d_u.cpu().numpy(), f)
+    a = ((f - prev).astype(np.float64) ** 2).sum()
+    b = (f.astype(np.float64) ** 2).sum()
+    assert np.float32(info[1]) == np.sqrt(np.float32(a)) / np.sqrt(np.float32(b))
