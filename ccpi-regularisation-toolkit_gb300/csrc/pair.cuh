@@ -5,8 +5,6 @@
 // those kernels.
 #pragma once
 
-#include <float.h>
-
 #include <type_traits>
 
 #include "runtime.cuh"
@@ -60,10 +58,11 @@ __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
 
 // sqrt(sq) and its reciprocal per component from one approximate reciprocal
 // square root: sqrt(sq) by Heron's step on sq rsqrt(sq), the reciprocal by
-// Newton's step, each within an ulp and issued paired.  FLT_MIN keeps sq = 0
-// finite (norm 0).
+// Newton's step, each within an ulp and issued paired.  The smallest subnormal
+// keeps sq = 0 finite (norm 0) and every other sq, subnormal or not, as it is:
+// images whose differences lie below 1e-19 shrink as larger ones do.
 __device__ __forceinline__ void norm2(float2 sq, float2& norm, float2& inverse) {
-    const float2 rs = make_float2(rsqrtf(fmaxf(sq.x, FLT_MIN)), rsqrtf(fmaxf(sq.y, FLT_MIN)));
+    const float2 rs = make_float2(rsqrtf(fmaxf(sq.x, 0x1p-149f)), rsqrtf(fmaxf(sq.y, 0x1p-149f)));
     norm = mul2(sq, rs);
     norm = fma2(mul2(splat(0.5f), rs), fma2(neg2(norm), norm, sq), norm);
     inverse = fma2(rs, fma2(neg2(norm), rs, splat(1.0f)), rs);
