@@ -116,14 +116,18 @@ int diff4th_run(const float* f, float* u_out, float lam, float sigma, int iters,
     CILREG_RANGE("cilreg Diff4th");
     const float sg2 = sigma * sigma;  // Diffus4th_order_core.c:51
     const float isg2 = 1.0f / sg2;    // den / sg2 formed as den * isg2 (within 1 ulp)
-    if (d4_strip_applies(d)) return d4_strip_run(f, u_out, lam, iters, tau, isg2, epsil, d, s, info);
+    // The kernels that hold pixel pairs form 1/(1 + den/sigma^2) by rcp2, which has no
+    // value above 2^126: a sigma so small that usual gradients get there runs the
+    // one-voxel kernel, whose IEEE reciprocal ends in 0.
+    const bool pairs = isg2 <= 0x1p64f;
+    if (pairs && d4_strip_applies(d)) return d4_strip_run(f, u_out, lam, iters, tau, isg2, epsil, d, s, info);
     const bool three = d.nz > 1;
     Scratch scratch(s);
     const Launch3 L = plan_launch(d);
     // CILREG_D4_KERNEL=simple selects the two per-voxel kernels (kept for A/B checks)
     const char* ek = getenv("CILREG_D4_KERNEL");
     const bool stream = !(ek && strcmp(ek, "simple") == 0);
-    const D4Plan T = d4_stream_plan(d);
+    const D4Plan T = d4_stream_plan(d, pairs);
     IterControl ctl(s, scratch, iters, epsil, stream ? T.nblocks : num_blocks(L));
     CILREG_TRY(ctl.status());
     float* W = scratch.floats(d.n);

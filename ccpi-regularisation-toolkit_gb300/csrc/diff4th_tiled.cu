@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(NT, 2) k_d4_stream(const float* __restrict__ U
 
 }  // namespace
 
-D4Plan d4_stream_plan(const Dims& d) {
-    if (d4_pair_applies(d)) return d4_pair_plan(d);
+D4Plan d4_stream_plan(const Dims& d, bool pairs) {
+    if (pairs && d4_pair_applies(d)) return d4_pair_plan(d);
     D4Plan T;
     T.block = dim3(BX, BY, 1);
     if (d.nz > 1) {

@@ -12,11 +12,11 @@ struct D4Plan {
     bool pair = false;  // the two-voxels-per-thread kernel (diff4th_pair.cu)
 };
 
-// the plan of the streaming kernel that runs for `d`: volumes of fewer than
+// the plan of the streaming kernel that runs for `d`: with `pairs`, volumes of fewer than
 // 2^31 voxels (rows of two voxels, or three and more) run k_d4_pair, images with
 // nx even k_d4_pair2d where they do not run strips (CILREG_D4_KERNEL=stream
 // selects k_d4_stream), others k_d4_stream
-D4Plan d4_stream_plan(const Dims& d);
+D4Plan d4_stream_plan(const Dims& d, bool pairs);
 bool d4_pair_applies(const Dims& d);
 D4Plan d4_pair_plan(const Dims& d);
 int d4_pair_step(const D4Plan& T, const float* cur, float* nxt, const float* f, float lam, float tau, float isg2,

@@ -860,3 +860,18 @@ def test_sb_shrinks_images_of_tiny_values(shape, monkeypatch):
     monkeypatch.setenv("CILREG_SB_KERNEL", "tiled")
     want = R.SB_TV(x, 0.03 * float(scale), 30).cpu().numpy()
     np.testing.assert_allclose(got, want, rtol=0, atol=1e-4 * float(np.ptp(want)))
+
+
+@pytest.mark.parametrize("shape", [(61, 91), (9, 33, 41), (61, 90), (9, 33, 40)])
+def test_diff4th_with_a_vanishing_edge_parameter(shape, monkeypatch):
+    """sigma so small that 1 + |grad U|^2 / sigma^2 overflows: its reciprocal is 0."""
+    import torch
+    from ccpi.filters import regularisersCuPy as R
+
+    rng = np.random.default_rng(14)
+    x = torch.from_numpy((rng.random(shape) * 255).astype(np.float32)).cuda()
+    got = R.Diff4th(x, 0.8, 1e-18, 12, 1e-4).cpu().numpy()
+    monkeypatch.setenv("CILREG_D4_KERNEL", "stream")
+    want = R.Diff4th(x, 0.8, 1e-18, 12, 1e-4).cpu().numpy()
+    assert np.isfinite(want).all()
+    np.testing.assert_array_equal(got, want)
