@@ -38,10 +38,16 @@ int held_arrays(int alg, bool three) {
     }
 }
 int transient_arrays(int alg, bool three) {
-    if (alg == ALG_FGP) return 1;
-    if (alg == ALG_SB) return 1 + (three ? 3 : 2);  // U ping-pong + B ping-pong
+    // 2D images run several iterations per launch between two sets of buffers:
+    // P and the P before it twice, and with a stopping rule a second U
+    // (fgp_strip.cu); U once and B twice (sb_strip.cu)
+    if (alg == ALG_FGP) return three ? 1 : 9;
+    if (alg == ALG_SB) return three ? 4 : 5;  // 3D: U ping-pong + B ping-pong
     return 2;
 }
+// the partial sums of a 2D run's checks: two sets of 16 bytes per tile, which
+// stores at least 32 x 14 pixels
+size_t partial_bytes(const Dims& d) { return d.nz > 1 ? 0 : arr_bytes(d) / 32; }
 
 __global__ void k_grad_step(float* __restrict__ z, const float* __restrict__ y, const float* __restrict__ f,
                             float step, long long n) {
@@ -181,7 +187,8 @@ extern "C" {
 long long cilreg_prox_session_bytes(int alg, int dimX, int dimY, int dimZ) {
     if (check_dims(dimX, dimY, dimZ) != 0 || alg < 0 || alg > 3) return -1;
     const Dims d = make_dims(dimX, dimY, dimZ < 1 ? 1 : dimZ);
-    return (long long)(arr_bytes(d) * (size_t)(held_arrays(alg, d.nz > 1) + transient_arrays(alg, d.nz > 1))) + (1 << 20);
+    return (long long)(arr_bytes(d) * (size_t)(held_arrays(alg, d.nz > 1) + transient_arrays(alg, d.nz > 1)) +
+                       partial_bytes(d)) + (1 << 20);
 }
 
 int cilreg_prox_session_create(cilreg_session** out, int alg, const float* params, int nparams, int dimX, int dimY,

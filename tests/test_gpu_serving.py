@@ -161,3 +161,35 @@ def test_cold_session_prox_equals_plain_call_and_state_persists(alg, prm):
     torch.cuda.synchronize()
     assert torch.equal(out1, plain)
     assert not torch.equal(out2, out1)  # the second prox started from the kept state
+
+
+@pytest.mark.parametrize("shape", [(1, 600, 500), (1, 1201, 1101), (33, 70, 81), (40, 96, 128)])
+@pytest.mark.parametrize("alg,prm", [(0, [0.02, 0.001]), (1, [0.05, 0, 0]), (2, [0.05, 0]), (3, [0.02, 0.05, 0.01, 1])])
+@pytest.mark.parametrize("tol", [0.0, 1e-9])
+def test_session_bytes_cover_a_prox_call(alg, prm, shape, tol):
+    """The reported size bounds what a session and its prox calls take from the
+    device's pool (the pool's own high-water mark)."""
+    import ctypes
+
+    import torch
+    from ccpi.filters.utils import cilregcuda as C
+
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64(0)
+    f = torch.rand(shape, device="cuda")
+    out = torch.zeros_like(f)
+    torch.cuda.synchronize()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0  # used now
+    before = used.value
+    used.value = 0
+    assert cu.cuMemPoolSetAttribute(pool, 8, ctypes.byref(used)) == 0  # restart the high-water mark
+    dims = shape[::-1]
+    s, h = torch.cuda.current_stream().cuda_stream, ctypes.c_void_p()
+    assert C.cilreg_prox_session_create(ctypes.byref(h), alg, (ctypes.c_float * 4)(*prm), len(prm), *dims, s) == 0
+    for _ in range(2):  # cold, then warm
+        assert C.cilreg_prox_session_prox(h, f.data_ptr(), out.data_ptr(), 40, tol, None, s) == 0
+    torch.cuda.synchronize()
+    assert C.cilreg_prox_session_destroy(h, s) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 8, ctypes.byref(used)) == 0
+    assert 0 < used.value - before <= C.cilreg_prox_session_bytes(alg, *dims)
