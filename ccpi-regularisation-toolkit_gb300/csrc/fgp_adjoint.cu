@@ -46,7 +46,7 @@ struct AdjArgs {
     const float* lam;     // per volume: lambda, then m
     double2* sums;        // per CTA: <Qbar_k, B U_k> and -<Zbar_k, A R_k> over all k
     float ck, a1, a2;
-    int nonneg, aniso, nvol;
+    int nonneg, aniso;
 };
 
 constexpr int BX = 32, BY = 20;
@@ -447,7 +447,6 @@ int fgp_vjp_run(const float* f, const float* ybar, const float* lams, int nvol, 
             a.a2 = cc[k + 2];
             a.nonneg = (nonneg == 1);
             a.aniso = (methodTV != 0);
-            a.nvol = nvol;
             auto kern = awide ? (three ? k_adj_stream<true, long long> : k_adj_stream<false, long long>)
                               : (three ? k_adj_stream<true, int> : k_adj_stream<false, int>);
             CILREG_CUDA(launch_pdl(kern, agrid, ablock, 0, s, a, d, azc, nchunk, kz));

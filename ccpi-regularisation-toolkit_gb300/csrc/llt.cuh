@@ -7,12 +7,6 @@
 
 namespace cilreg {
 
-__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
-    const float2 m = make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
-                                 fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
-    return pair::mul2(m, m);
-}
-
 // dp / sqrt(s) per component
 __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
     return pair::mul2(dp, make_float2(rsqrtf(s.x), rsqrtf(s.y)));

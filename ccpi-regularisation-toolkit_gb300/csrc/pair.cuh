@@ -56,6 +56,17 @@ __device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
     return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
 }
 
+// minmod(a, b) per component up to its sign (ROF_TV_core.c:132): the median of
+// a, b and 0 has its magnitude; and its square
+__device__ __forceinline__ float2 minmod2(float2 a, float2 b) {
+    return make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
+                       fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
+}
+__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
+    const float2 m = minmod2(a, b);
+    return mul2(m, m);
+}
+
 // sqrt(sq) and its reciprocal per component from one approximate reciprocal
 // square root: sqrt(sq) by Heron's step on sq rsqrt(sq), the reciprocal by
 // Newton's step, each within an ulp and issued paired.  The smallest subnormal

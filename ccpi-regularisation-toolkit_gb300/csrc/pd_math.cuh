@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "pair.cuh"
 
 namespace cilreg {
 
@@ -41,6 +42,16 @@ __device__ __forceinline__ float div_by_double(float num, const DoubleDivisor& D
     float r = __fmaf_rn(-q, D.hi, num);
     r = __fsub_rn(r, __fmul_rn(q, D.lo));
     return __fmaf_rn(r, D.rcp, q);
+}
+
+// the same for a pixel pair, additions paired
+__device__ __forceinline__ float2 div_by_double2(float2 num, const DoubleDivisor& D) {
+    using namespace pair;
+    const float2 rcp = splat(D.rcp);
+    const float2 q = mul2_rn(num, rcp);
+    float2 r = fma2(neg2(q), splat(D.hi), num);
+    r = sub2(r, mul2_rn(q, splat(D.lo)));
+    return fma2(r, rcp, q);
 }
 
 // P + sigma (Ue[+1] - Ue)  (PD_TV_core.c:222-227)

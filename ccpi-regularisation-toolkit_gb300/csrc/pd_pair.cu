@@ -40,14 +40,6 @@ constexpr int OYD = ROWS - 2;
 constexpr int NTD = LX * ROWS, TPD = 2 * NTD;
 constexpr int ZCHUNK = 64;
 
-__device__ __forceinline__ float2 div2(float2 num, const DoubleDivisor& D) {
-    const float2 rcp = splat(D.rcp);
-    const float2 q = mul2_rn(num, rcp);
-    float2 r = fma2(neg2(q), splat(D.hi), num);
-    r = sub2(r, mul2_rn(q, splat(D.lo)));
-    return fma2(r, rcp, q);
-}
-
 template <bool CHECK, bool ALIGNED>
 __global__ void __launch_bounds__(NTD, 4) k_pd_pair(PdStreamArgs a, Dims d, int zc, const StopCtl* ctl,
                                                     double2* partials) {
@@ -157,7 +149,7 @@ __global__ void __launch_bounds__(NTD, 4) k_pd_pair(PdStreamArgs a, Dims d, int 
             float2 uc = um1;
             if (a.nonneg) uc = make_float2(uc.x < 0.f ? 0.f : uc.x, uc.y < 0.f ? 0.f : uc.y);
             const float2 num = add2(sub2(uc, mul2_rn(tau2, dv)), mul2_rn(lt2, fq));
-            const float2 un = div2(num, a.onelt);
+            const float2 un = div_by_double2(num, a.onelt);
             const int v = k * sxy + col;
             if (CHECK) {
                 const float2 df = sub2(un, uc);

@@ -26,14 +26,6 @@ struct Args {
     bool nonneg, aniso;
 };
 
-__device__ __forceinline__ float2 div2(float2 num, const DoubleDivisor& D) {
-    const float2 rcp = splat(D.rcp);
-    const float2 q = mul2_rn(num, rcp);
-    float2 r = fma2(neg2(q), splat(D.hi), num);
-    r = sub2(r, mul2_rn(q, splat(D.lo)));
-    return fma2(r, rcp, q);
-}
-
 template <int R, bool CHECK>
 __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame fr) {
     __shared__ float2 firstU[NW][32], lastU[NW][32], lastP[NW][32];
@@ -100,7 +92,7 @@ __global__ void __launch_bounds__(NT, R <= 3 ? 2 : 1) k_pd_strip2d(Args a, Frame
             const float2 dv = add2(sub2(make_float2(lo, p1[r].x), p1[r]), sub2(p2up, p2[r]));
             float2 uc = u[r];
             if (a.nonneg) uc = make_float2(uc.x < 0.f ? 0.f : uc.x, uc.y < 0.f ? 0.f : uc.y);
-            const float2 un = div2(add2(sub2(uc, mul2_rn(tau2, dv)), ltf[r]), a.onelt);
+            const float2 un = div_by_double2(add2(sub2(uc, mul2_rn(tau2, dv)), ltf[r]), a.onelt);
             if (CHECK && sum) {
                 add_norms(q, r, un, uc, norms);
                 q.store(a.brk, r, un);

@@ -54,17 +54,6 @@ struct Geo {
     static constexpr size_t SMEM = sizeof(float) * TP * (RING + 4);  // U ring, D1 and D2 (two planes each)
 };
 
-// minmod(a, b) per component up to its sign (ROF_TV_core.c:132): the median of
-// a, b and 0 has its magnitude; and its square
-__device__ __forceinline__ float2 minmod2(float2 a, float2 b) {
-    return make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
-                       fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
-}
-__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
-    const float2 m = minmod2(a, b);
-    return mul2(m, m);
-}
-
 // dp / sqrt(s) per component, one reciprocal square root each
 __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {
     return mul2(dp, make_float2(rsqrtf(s.x), rsqrtf(s.y)));

@@ -14,12 +14,6 @@ namespace {
 
 using namespace strip;
 
-__device__ __forceinline__ float2 minmod_sq2(float2 a, float2 b) {
-    const float2 m = make_float2(fmaxf(fminf(a.x, b.x), fminf(fmaxf(a.x, b.x), 0.f)),
-                                 fmaxf(fminf(a.y, b.y), fminf(fmaxf(a.y, b.y), 0.f)));
-    return mul2(m, m);
-}
-
 // ONCE: the result is only used by one subtraction
 template <bool ONCE = false>
 __device__ __forceinline__ float2 normalise2(float2 dp, float2 s) {

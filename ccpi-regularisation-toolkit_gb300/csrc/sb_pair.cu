@@ -43,30 +43,6 @@ constexpr int LX = 16;
 constexpr int OXS = 2 * LX - 4;
 constexpr int ZCHUNK = 64;
 
-// D = shrink(g + b) and B = b + (g - D) of a pair (SB_TV_core.c:284-371)
-template <bool ANISO>
-__device__ __forceinline__ void shrink(const float2 (&g)[3], const float2 (&b)[3], float dlam, float2 (&dd)[3],
-                                       float2 (&n)[3]) {
-    float2 v[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) v[c] = add2(g[c], b[c]);
-    if (ANISO) {
-        // (v / |v|) * max(|v| - 1/lambda, 0), 0 for v == 0: the same value as a sign copy
-        auto one = [&](float x) { return copysignf(fmaxf(fabsf(x) - dlam, 0.f), x); };
-#pragma unroll
-        for (int c = 0; c < 3; c++) dd[c] = make_float2(one(v[c].x), one(v[c].y));
-    } else {
-        const float2 sq = fma2(v[2], v[2], fma2(v[0], v[0], mul2(v[1], v[1])));
-        float2 den, r;
-        norm2(sq, den, r);
-        const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
-#pragma unroll
-        for (int c = 0; c < 3; c++) dd[c] = mul2(m, mul2(v[c], r));
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) n[c] = add2(b[c], sub2(g[c], dd[c]));
-}
-
 template <bool CHECK, bool ANISO, bool ALIGNED, int ROWS>
 __global__ void __launch_bounds__(LX * ROWS, 2) k_sb_pair(SbFusedArgs a, Dims d, int zc, const StopCtl* ctl,
                                                           double2* partials) {
@@ -158,7 +134,7 @@ __global__ void __launch_bounds__(LX * ROWS, 2) k_sb_pair(SbFusedArgs a, Dims d,
             const int m0 = j - 1;
             const float2 zhi = (m0 == nz - 1) ? ppu : cu;  // mirrored k+1 (SB_TV_core.c:293)
             const float2 gr[3] = {sub2(above(pu), pu), sub2(ld2(sU[SM1] + oyh), pu), sub2(zhi, pu)};
-            shrink<ANISO>(gr, cb, dlam, da, ba);
+            sb_shrink2(gr, cb, dlam, ANISO, da, ba);
             if (upd && m0 >= z0 && m0 < z1) {
                 const int v = m0 * sxy + col;
 #pragma unroll

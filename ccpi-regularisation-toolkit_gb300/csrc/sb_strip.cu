@@ -24,27 +24,16 @@ struct Args {
     bool aniso;
 };
 
-// D = shrink(g + b) and B = b + (g - D) of a pair, as D - B and B
+// D - B and B of a pair after a shrinkage
 __device__ __forceinline__ void shrink(float2 g1, float2 g2, float2 b1, float2 b2, float dlam, bool aniso, float2& q1,
                                        float2& q2, float2& n1, float2& n2) {
-    const float2 v1 = add2(g1, b1), v2 = add2(g2, b2);
-    float2 d1, d2;
-    if (aniso) {
-        // (v / |v|) * max(|v| - 1/lambda, 0), 0 for v == 0: the same value as a sign copy
-        auto one = [&](float v) { return copysignf(fmaxf(fabsf(v) - dlam, 0.f), v); };
-        d1 = make_float2(one(v1.x), one(v1.y));
-        d2 = make_float2(one(v2.x), one(v2.y));
-    } else {
-        float2 den, r;
-        pair::norm2(fma2(v1, v1, mul2(v2, v2)), den, r);
-        const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
-        d1 = mul2(m, mul2(v1, r));
-        d2 = mul2(m, mul2(v2, r));
-    }
-    n1 = add2(b1, sub2(g1, d1));
-    n2 = add2(b2, sub2(g2, d2));
-    q1 = sub2(d1, n1);
-    q2 = sub2(d2, n2);
+    const float2 g[2] = {g1, g2}, b[2] = {b1, b2};
+    float2 d[2], n[2];
+    sb_shrink2(g, b, dlam, aniso, d, n);
+    n1 = n[0];
+    n2 = n[1];
+    q1 = sub2(d[0], n[0]);
+    q2 = sub2(d[1], n[1]);
 }
 
 template <int R, bool CHECK>

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "drivers.cuh"
+#include "pair.cuh"
 #include "runtime.cuh"
 
 namespace cilreg {
@@ -26,6 +27,33 @@ struct SbFusedArgs {
     float* bn[3];          // B^k (distinct buffers: a neighbouring tile still reads B^{k-1})
     float lambda, mu, norm, dlam;
 };
+
+// D = shrink(g + b) and B = b + (g - D) of a voxel pair's N components
+// (SB_TV_core.c:284-371)
+template <int N>
+__device__ __forceinline__ void sb_shrink2(const float2 (&g)[N], const float2 (&b)[N], float dlam, bool aniso,
+                                           float2 (&dd)[N], float2 (&n)[N]) {
+    using namespace pair;
+    float2 v[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) v[c] = add2(g[c], b[c]);
+    if (aniso) {
+        // (v / |v|) * max(|v| - 1/lambda, 0), 0 for v == 0: the same value as a sign copy
+        auto one = [&](float x) { return copysignf(fmaxf(fabsf(x) - dlam, 0.f), x); };
+#pragma unroll
+        for (int c = 0; c < N; c++) dd[c] = make_float2(one(v[c].x), one(v[c].y));
+    } else {
+        float2 sq = fma2(v[0], v[0], mul2(v[1], v[1]));
+        if (N > 2) sq = fma2(v[N - 1], v[N - 1], sq);
+        float2 den, r;
+        norm2(sq, den, r);
+        const float2 m = make_float2(fmaxf(den.x - dlam, 0.f), fmaxf(den.y - dlam, 0.f));
+#pragma unroll
+        for (int c = 0; c < N; c++) dd[c] = mul2(m, mul2(v[c], r));
+    }
+#pragma unroll
+    for (int c = 0; c < N; c++) n[c] = add2(b[c], sub2(g[c], dd[c]));
+}
 
 struct SbPlan {
     dim3 grid, block;
