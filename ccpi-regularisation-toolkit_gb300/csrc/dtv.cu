@@ -4,10 +4,10 @@
 // Once per call the eta-smoothed unit gradient field B of the reference image
 // is formed (GradNorm_func, FGP_dTV_core.c:273-300).  Each iteration then is
 // the FGP iteration with R and the gradient of U projected onto the
-// orthogonal complement of B at every voxel; it runs on the FGP streaming
-// kernel's dTV variant (fgp_tiled.cu): one launch per iteration reading
-// P^{k-1}, P^{k-2}, f and B and writing P^k (52 B per voxel in 3D), R and U
-// never stored.  The momentum recurrence and the stopping rule are FGP's;
+// orthogonal complement of B at every voxel.  2D images run several iterations
+// per launch (fgp_strip.cu), volumes the FGP streaming kernel's dTV variant
+// (fgp_tiled.cu): one launch per iteration reading P^{k-1}, P^{k-2}, f and B and
+// writing P^k (52 B per voxel), R and U never stored.  The momentum recurrence and the stopping rule are FGP's;
 // t_{k+1} is formed with a double square root as the reference does.
 #include <math.h>
 
@@ -61,8 +61,8 @@ int dtv_run(const float* f, const float* ref, float* u_out, float lam, int iters
     const bool three = d.nz > 1;
     const int nc = three ? 3 : 2;
     Scratch scratch(s);
-    // 2D images with an even row length: the two-pixel kernel; otherwise the
-    // streaming kernel (whatever CILREG_FGP_KERNEL says, bar 'stream')
+    // volumes, and images that do not run strips: the streaming kernel, or the
+    // two-pixel kernel where rows are even (bar CILREG_FGP_KERNEL=stream)
     TiledPlan T = fgp_tiled_plan(d, 2);  // two CTAs of the dTV instantiation per SM
     if (d.nz == 1) {
         const TiledPlan X = fgp_x2_plan(d);
